@@ -1840,7 +1840,8 @@ extern "C" pico_status pico_gpu_autotune(pico_ctx* ctx, pico_field field, uint32
     in_words = std::max<uint64_t>(in_words, (uint64_t)width_for(l) << l);
     out_words = std::max<uint64_t>(out_words, (uint64_t)width_for(l) << (l + 1));
   }
-  const uint64_t hash_rows = 1u << 20, hash_w = 64;
+  // launches of kTcMinStates rows on take no block size
+  const uint64_t hash_rows = kTcMinStates / 2, hash_w = 64;
   out_words = std::max<uint64_t>(out_words, hash_rows * hash_w);
   const uint64_t need = (2 * in_words + 2 * out_words + 2 * kPwWords + hash_rows * 8) * 4;
   if (!try_reserve(ctx, need)) {

@@ -28,6 +28,12 @@ struct RowGroup {
 // --- Poseidon2 / Merkle kernels (p2_kernels.cu) -------------------------
 cudaError_t upload_p2_constants(int field, const uint32_t ext[8][16], const uint32_t* inte, int rounds_p,
                                 const uint32_t diag[16]);
+// Launches of at least this many states use the tensor-core form (p2_tc.cuh).
+// One permutation of n states, one thread per state against the tensor cores
+// (KoalaBear, host call included): 2^15 23.8 / 29.1 us, 2^16 31.2 / 29.3,
+// 2^17 46.2 / 39.1, 2^20 226 / 160.  Below, the latency of one permutation
+// sets the time, and the table load and product stages make it longer.
+constexpr uint64_t kTcMinStates = 1u << 16;
 // four_lanes: four threads per state (the latency form).
 cudaError_t launch_permute(int field, uint32_t* states, uint64_t n, cudaStream_t st, bool four_lanes = false);
 // Levels of at most this many nodes are compressed four threads per node.
@@ -85,6 +91,7 @@ enum GuardTag : int {
   kGuardLoad = 1,       // LDE global load (offset / extent in words of the pass's input)
   kGuardStore = 2,      // LDE global store (offset / extent in words of the pass's output)
   kGuardRowRead = 10,   // row hashing: segment index / column
+  kGuardTensorWait = 11,  // tensor-core Poseidon2: a wait for a product ran out
   kGuardTile = 100,     // LDE shared-memory tile index
   kGuardTwiddle = 101,  // LDE shared-memory twiddle index
   kGuardPowIndex = 102  // coset power-table exponent

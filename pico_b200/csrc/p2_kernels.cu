@@ -3,9 +3,14 @@
 // FRI fold, and the device-side duplex challenger.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <cstring>
+#include <vector>
+
 #include "field.cuh"
 #include "internal.h"
 #include "open.h"
+#include "p2_tc.cuh"
 #include "poseidon2.cuh"
 
 namespace pico {
@@ -17,7 +22,13 @@ cudaError_t upload_p2_constants(int field, const uint32_t ext[8][16], const uint
     for (int j = 0; j < 16; j++) h.ext[r][j] = ext[r][j];
   for (int r = 0; r < rounds_p && r < 24; r++) h.inte[r] = inte[r];
   for (int j = 0; j < 16; j++) h.diag[j] = diag[j];
-  return cudaMemcpyToSymbol(c_p2, &h, sizeof h, sizeof(P2Constants) * (field ? 1 : 0));
+  cudaError_t e = cudaMemcpyToSymbol(c_p2, &h, sizeof h, sizeof(P2Constants) * (field ? 1 : 0));
+  if (e) return e;
+  std::vector<uint8_t> tables(kTcTableBytes);
+  P2TcConstants tc;
+  build_p2_tc_tables(field, h.ext, h.inte, h.diag, tables.data(), &tc);
+  if ((e = cudaMemcpyToSymbol(g_p2_tc, tables.data(), kTcTableBytes, (size_t)kTcTableBytes * (field ? 1 : 0)))) return e;
+  return cudaMemcpyToSymbol(c_p2_tc, &tc, sizeof tc, sizeof tc * (field ? 1 : 0));
 }
 
 // ---------------------------------------------------------------------------
@@ -50,9 +61,10 @@ __global__ void k_permute(uint32_t* states, uint64_t n) {
 // g_hash_guard, and reported by the entry points after their final
 // synchronisation.
 __device__ GuardRecord g_hash_guard;
-__device__ __forceinline__ void hash_guard_trip(unsigned long long seg, unsigned long long col) {
+__device__ __forceinline__ void hash_guard_trip(unsigned long long seg, unsigned long long col,
+                                                unsigned long long tag = kGuardRowRead) {
   if (atomicAdd(&g_hash_guard.count, 1ull) == 0) {
-    g_hash_guard.tag = kGuardRowRead;
+    g_hash_guard.tag = tag;
     g_hash_guard.offset = seg;
     g_hash_guard.extent = col;
     g_hash_guard.block = blockIdx.x;
@@ -240,6 +252,250 @@ __global__ void __launch_bounds__(256)
 }
 
 // ---------------------------------------------------------------------------
+// Tensor-core forms (p2_tc.cuh): 128 states per CTA of 128 threads, four CTAs
+// per SM (their 4 x 128 TMEM columns).
+
+// The next up to 8 columns of row r: words of chunk positions [lo, hi) into
+// v, through the segment cursor (seg, col, segw, rowp).
+struct RowCursor {
+  uint32_t seg, col, segw;
+  const uint32_t* rowp;
+};
+__device__ __forceinline__ void row_cursor_begin(RowCursor& c, const RowSeg* segs, uint32_t n_segs, uint64_t r) {
+  c.seg = c.col = 0;
+  c.segw = n_segs ? segs[0].width : 0u;
+  c.rowp = n_segs ? segs[0].ptr + r * c.segw : nullptr;
+}
+__device__ __forceinline__ void row_chunk(RowCursor& c, const RowSeg* segs, uint32_t n_segs, uint64_t r, int lo, int hi,
+                                          uint32_t v[8]) {
+  if (lo == 0 && hi == 8 && c.segw - c.col >= 8) {
+#pragma unroll
+    for (int j = 0; j < 8; j++) v[j] = __ldg(c.rowp + c.col + j);
+    c.col += 8;
+    return;
+  }
+#pragma unroll
+  for (int j = 0; j < 8; j++) {
+    if (j >= lo && j < hi) {
+      while (c.col == c.segw && c.seg < n_segs) {
+        c.seg++;
+        c.col = 0;
+        c.segw = c.seg < n_segs ? segs[c.seg].width : 0u;
+        c.rowp = c.seg < n_segs ? segs[c.seg].ptr + r * c.segw : nullptr;
+      }
+      if (c.seg >= n_segs) {
+        hash_guard_trip(c.seg, c.col);
+        v[j] = 0;
+      } else {
+        v[j] = __ldg(c.rowp + c.col);
+      }
+      c.col++;
+    }
+  }
+}
+
+__host__ __device__ static inline uint64_t tc_tiles(uint64_t n) { return (n + kTcThreads - 1) / kTcThreads; }
+#define PICO_TC_OPEN(F)                                  \
+  extern __shared__ __align__(128) uint8_t tc_tables[];  \
+  __shared__ __align__(8) uint64_t tc_bar[kTcGroups];    \
+  __shared__ uint32_t tc_slot;                           \
+  P2Tc<F> tc;                                            \
+  tc.open(tc_tables, tc_bar, &tc_slot)
+#define PICO_TC_CLOSE()                                          \
+  tc.close();                                                    \
+  if (tc.dead) hash_guard_trip(0, 0, kGuardTensorWait)
+
+template <class F>
+__global__ void __launch_bounds__(kTcThreads * kTcGroups, kTcCtas) k_permute_tc(uint32_t* states, uint64_t n) {
+  PICO_TC_OPEN(F);
+  for (uint64_t t0 = tc.first_tile(tc_tiles(n)) * kTcThreads; t0 < n; t0 += tc.tile_stride() * kTcThreads) {
+    const uint64_t i = t0 + threadIdx.x % kTcThreads;
+    uint32_t s[16];
+    uint4* p = reinterpret_cast<uint4*>(states + 16 * (i < n ? i : n - 1));
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const uint4 v = p[k];
+      s[4 * k] = v.x;
+      s[4 * k + 1] = v.y;
+      s[4 * k + 2] = v.z;
+      s[4 * k + 3] = v.w;
+    }
+    tc.put_state(s);
+    tc.body(kTcFromState);
+    tc.output(s);
+    if (i < n) {
+#pragma unroll
+      for (int k = 0; k < 4; k++) p[k] = make_uint4(s[4 * k], s[4 * k + 1], s[4 * k + 2], s[4 * k + 3]);
+    }
+  }
+  PICO_TC_CLOSE();
+}
+
+// Row digests of a GroupBatch (k_hash_groups' sponges).  Tiles of 128 rows do
+// not cross groups, so a CTA's rows have one width.
+template <class F>
+__global__ void __launch_bounds__(kTcThreads * kTcGroups, kTcCtas) k_hash_groups_tc(const __grid_constant__ GroupBatch b, uint64_t tiles_all) {
+  PICO_TC_OPEN(F);
+  uint64_t tile = tc.first_tile(tiles_all);
+  uint32_t g = 0;
+  uint64_t row0 = 0, first = 0;  // of group g: its first global row, its first tile
+  const uint32_t n_groups = b.n_groups <= (uint32_t)kBatchGroups ? b.n_groups : 0u;
+  for (; g < n_groups;) {
+    const uint64_t rows = b.row_end[g] - row0, tiles = (rows + kTcThreads - 1) / kTcThreads;
+    if (tile >= first + tiles) {
+      first += tiles;
+      row0 = b.row_end[g];
+      g++;
+      continue;
+    }
+    const uint64_t r = (tile - first) * kTcThreads + threadIdx.x % kTcThreads;
+    const uint64_t rr = r < rows ? r : rows - 1;
+    const uint32_t s0 = b.seg_begin[g], s1 = b.seg_begin[g + 1], W = b.width[g];
+    uint32_t s[16];
+#pragma unroll
+    for (int k = 0; k < 16; k++) s[k] = 0;
+    if (s1 < s0 || s1 > (uint32_t)kBatchSegs) {
+      hash_guard_trip(s0, s1);
+    } else {
+      const RowSeg* segs = b.segs + s0;
+      RowCursor cur;
+      row_cursor_begin(cur, segs, s1 - s0, rr);
+      for (uint32_t base = 0; base < W; base += 8) {
+        const int hi = W - base < 8 ? (int)(W - base) : 8;
+        TcInput from = base ? kTcFromSponge : kTcFromRate;
+        if (base && hi < 8) {  // a partial chunk keeps the other rate words: through registers
+          tc.output(s);
+          from = kTcFromState;
+        }
+        row_chunk(cur, segs, s1 - s0, rr, 0, hi, s);
+        if (from == kTcFromState)
+          tc.put_state(s);
+        else
+          tc.put_rate(s);
+        tc.body(from);
+      }
+      if (W) tc.digest(s);
+    }
+    if (r < rows) store_digest(b.out[g] + 8 * r, s);
+    tile += tc.tile_stride();
+  }
+  PICO_TC_CLOSE();
+}
+
+// k_absorb_rows on the tensor cores.
+template <class F>
+__global__ void __launch_bounds__(kTcThreads * kTcGroups, kTcCtas)
+    k_absorb_rows_tc(const __grid_constant__ RowGroup g, uint64_t rows, uint32_t pos0, const uint32_t* state_in,
+                     uint32_t* state_out, uint32_t* digest_out) {
+  PICO_TC_OPEN(F);
+  for (uint64_t t0 = tc.first_tile(tc_tiles(rows)) * kTcThreads; t0 < rows; t0 += tc.tile_stride() * kTcThreads) {
+    const uint64_t r = t0 + threadIdx.x % kTcThreads, rr = r < rows ? r : rows - 1;
+    uint32_t s[16];
+    if (state_in) {
+      const uint4* p = reinterpret_cast<const uint4*>(state_in + 16 * rr);
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const uint4 v = p[k];
+        s[4 * k] = v.x;
+        s[4 * k + 1] = v.y;
+        s[4 * k + 2] = v.z;
+        s[4 * k + 3] = v.w;
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < 16; k++) s[k] = 0;
+    }
+    const int end = (int)(pos0 + g.total_width);
+    bool held = true;  // the state is in s (else its last S-boxes are in TMEM)
+    RowCursor cur;
+    row_cursor_begin(cur, g.segs, g.n_segs, rr);
+    for (int base = 0; base < end; base += 8) {
+      const int lo = base < (int)pos0 ? (int)pos0 - base : 0, hi = end - base < 8 ? end - base : 8;
+      const bool permute = base + 8 <= end || digest_out;
+      const bool full = lo == 0 && hi == 8;
+      if (!held && !full) {
+        tc.output(s);
+        held = true;
+      }
+      row_chunk(cur, g.segs, g.n_segs, rr, lo, hi, s);
+      if (!permute) break;
+      if (held)
+        tc.put_state(s);
+      else
+        tc.put_rate(s);
+      tc.body(held ? kTcFromState : kTcFromSponge);
+      held = false;
+    }
+    if (digest_out) {
+      if (!held) tc.digest(s);
+      if (r < rows) store_digest(digest_out + 8 * r, s);
+    } else {
+      if (!held) tc.output(s);
+      if (r < rows) {
+        uint4* o = reinterpret_cast<uint4*>(state_out + 16 * r);
+#pragma unroll
+        for (int k = 0; k < 4; k++) o[k] = make_uint4(s[4 * k], s[4 * k + 1], s[4 * k + 2], s[4 * k + 3]);
+      }
+    }
+  }
+  PICO_TC_CLOSE();
+}
+
+// k_compress on the tensor cores.
+template <class F>
+__global__ void __launch_bounds__(kTcThreads * kTcGroups, kTcCtas)
+    k_compress_tc(const uint32_t* prev, uint32_t* next, uint64_t n, const uint32_t* inj) {
+  PICO_TC_OPEN(F);
+  for (uint64_t t0 = tc.first_tile(tc_tiles(n)) * kTcThreads; t0 < n; t0 += tc.tile_stride() * kTcThreads) {
+    const uint64_t i = t0 + threadIdx.x % kTcThreads, ii = i < n ? i : n - 1;
+    uint32_t s[16];
+    const uint4* p = reinterpret_cast<const uint4*>(prev + 16 * ii);
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const uint4 v = __ldg(p + k);
+      s[4 * k] = v.x;
+      s[4 * k + 1] = v.y;
+      s[4 * k + 2] = v.z;
+      s[4 * k + 3] = v.w;
+    }
+    for (int pass = 0;; pass++) {
+      tc.put_state(s);
+      tc.body(kTcFromState);
+      tc.digest(s);
+      if (!inj || pass) break;
+      const uint4* q = reinterpret_cast<const uint4*>(inj + 8 * ii);
+      const uint4 a = __ldg(q), c = __ldg(q + 1);
+      s[8] = a.x;
+      s[9] = a.y;
+      s[10] = a.z;
+      s[11] = a.w;
+      s[12] = c.x;
+      s[13] = c.y;
+      s[14] = c.z;
+      s[15] = c.w;
+    }
+    if (i < n) store_digest(next + 8 * i, s);
+  }
+  PICO_TC_CLOSE();
+}
+
+// Row hashing takes a CTA per kTcGroups tiles from this many permutations a
+// row on: the hardware then balances groups of different widths, and the
+// set-up (tables of 58 KB into shared memory, ~2 us) is a small part.
+constexpr uint64_t kTcWholeChunks = 4;
+// Launch a tensor-core kernel over `tiles` tiles: a full wave of CTAs, each
+// looping over its share, or (whole) a CTA per kTcGroups tiles.
+template <class... P, class... A>
+static cudaError_t tc_launch(void (*kernel)(P...), uint64_t tiles, bool whole, cudaStream_t st, A... args) {
+  uint64_t ctas = tiles;
+  if (ctas > kTcResident) ctas = whole ? std::max<uint64_t>((tiles + kTcGroups - 1) / kTcGroups, kTcResident) : kTcResident;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmemBytes);
+  if (e) return e;
+  kernel<<<(unsigned)ctas, kTcThreads * kTcGroups, kTcSmemBytes, st>>>(args...);
+  return cudaGetLastError();
+}
+
+// ---------------------------------------------------------------------------
 static inline unsigned blocks_for(uint64_t n, unsigned bs) { return (unsigned)((n + bs - 1) / bs); }
 
 // Four threads per state (the latency form).  Every thread of a launched warp
@@ -271,6 +527,10 @@ cudaError_t launch_permute(int field, uint32_t* states, uint64_t n, cudaStream_t
       k_permute_quad<BabyBear><<<blocks_for(4 * n, 256), 256, 0, st>>>(states, n);
     return cudaGetLastError();
   }
+  if (n >= kTcMinStates) {
+    return tc_launch(field == 0 ? k_permute_tc<KoalaBear> : k_permute_tc<BabyBear>, tc_tiles(n), false, st, states,
+                     n);
+  }
   if (field == 0)
     k_permute<KoalaBear><<<blocks_for(n, 256), 256, 0, st>>>(states, n);
   else
@@ -290,6 +550,18 @@ cudaError_t hash_guard_clear() {
 cudaError_t launch_hash_rows(int field, const RowGroup& g, uint64_t rows, uint32_t* out, cudaStream_t st,
                              unsigned block) {
   if (rows == 0) return cudaSuccess;
+  if (rows >= kTcMinStates) {
+    GroupBatch b;
+    memset(&b, 0, sizeof b);
+    b.n_groups = 1;
+    b.n_segs = g.n_segs;
+    b.row_end[0] = rows;
+    b.out[0] = out;
+    b.seg_begin[1] = g.n_segs;
+    b.width[0] = g.total_width;
+    for (uint32_t k = 0; k < g.n_segs; k++) b.segs[k] = g.segs[k];
+    return launch_hash_groups(field, b, st, block);
+  }
   if (block < 32 || block > 256) block = 256;
   if (field == 0)
     k_hash_rows<KoalaBear><<<blocks_for(rows, block), block, 0, st>>>(g, rows, out);
@@ -303,6 +575,16 @@ cudaError_t launch_hash_groups(int field, const GroupBatch& b, cudaStream_t st, 
   if (b.n_groups > (uint32_t)kBatchGroups || b.n_segs > (uint32_t)kBatchSegs) return cudaErrorInvalidValue;
   const uint64_t rows = b.row_end[b.n_groups - 1];
   if (rows == 0) return cudaSuccess;
+  if (rows >= kTcMinStates) {
+    uint64_t tiles = 0, chunks = 0;
+    for (uint32_t g = 0; g < b.n_groups; g++) {
+      const uint64_t t = tc_tiles(b.row_end[g] - (g ? b.row_end[g - 1] : 0ull));
+      tiles += t;
+      chunks += t * ((b.width[g] + 7) / 8);
+    }
+    return tc_launch(field == 0 ? k_hash_groups_tc<KoalaBear> : k_hash_groups_tc<BabyBear>, tiles,
+                     chunks >= kTcWholeChunks * tiles, st, b, tiles);
+  }
   if (block < 32 || block > 256) block = 256;
   if (field == 0)
     k_hash_groups<KoalaBear><<<blocks_for(rows, block), block, 0, st>>>(b);
@@ -314,6 +596,10 @@ cudaError_t launch_hash_groups(int field, const GroupBatch& b, cudaStream_t st, 
 cudaError_t launch_absorb_rows(int field, const RowGroup& g, uint64_t rows, uint32_t pos0, const uint32_t* state_in,
                                uint32_t* state_out, uint32_t* digest_out, cudaStream_t st, unsigned block) {
   if (rows == 0) return cudaSuccess;
+  if (rows >= kTcMinStates) {
+    return tc_launch(field == 0 ? k_absorb_rows_tc<KoalaBear> : k_absorb_rows_tc<BabyBear>, tc_tiles(rows), pos0 + g.total_width >= 8 * kTcWholeChunks, st,
+                     g, rows, pos0, state_in, state_out, digest_out);
+  }
   if (block < 32 || block > 256) block = 256;
   if (field == 0)
     k_absorb_rows<KoalaBear><<<blocks_for(rows, block), block, 0, st>>>(g, rows, pos0, state_in, state_out,
@@ -363,6 +649,10 @@ cudaError_t launch_compress(int field, const uint32_t* prev, uint32_t* next, uin
     else
       k_compress_quad<BabyBear><<<blocks_for(4 * n_next, 256), 256, 0, st>>>(prev, next, n_next, inj_digests);
     return cudaGetLastError();
+  }
+  if (n_next >= kTcMinStates) {
+    return tc_launch(field == 0 ? k_compress_tc<KoalaBear> : k_compress_tc<BabyBear>, tc_tiles(n_next), false, st,
+                     prev, next, n_next, inj_digests);
   }
   if (field == 0)
     k_compress<KoalaBear><<<blocks_for(n_next, 256), 256, 0, st>>>(prev, next, n_next, inj_digests);
@@ -482,11 +772,51 @@ __global__ void __launch_bounds__(256) k_fri_fold_hash_rows(const uint32_t* cw, 
   lp[1] = make_uint4(s[4], s[5], s[6], s[7]);
 }
 
+// k_fri_fold_hash and k_fri_fold_hash_rows with the leaves hashed on the
+// tensor cores (p2_tc.cuh).
+template <class F>
+__global__ void __launch_bounds__(kTcThreads * kTcGroups, kTcCtas)
+    k_fri_fold_hash_tc(const uint32_t* cw, uint32_t log_len, uint64_t row0, uint64_t n_leaves, const uint32_t* beta,
+                       const __grid_constant__ TwiddleTables tw, uint32_t* out, const uint32_t* inject,
+                       uint32_t* leaves) {
+  PICO_TC_OPEN(F);
+  for (uint64_t t0 = tc.first_tile(tc_tiles(n_leaves)) * kTcThreads; t0 < n_leaves; t0 += tc.tile_stride() * kTcThreads) {
+    const uint64_t k = t0 + threadIdx.x % kTcThreads;
+    uint32_t s[8];
+    if (k < n_leaves) {
+      const Ext4 hb = half_beta<F>(beta);
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+        const uint64_t r = 2 * k + u;
+        Ext4 res = fri_fold_row<F>(cw, log_len, r, hb, tw, row0 + r);
+        if (inject) {
+          const uint4 v = __ldg(reinterpret_cast<const uint4*>(inject) + r);
+          res = Ef<F>::add(res, Ext4{{v.x, v.y, v.z, v.w}});
+        }
+        reinterpret_cast<uint4*>(out)[r] = make_uint4(res.c[0], res.c[1], res.c[2], res.c[3]);
+#pragma unroll
+        for (int i = 0; i < 4; i++) s[4 * u + i] = res.c[i];
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; i++) s[i] = 0;
+    }
+    tc.put_rate(s);
+    tc.body(kTcFromRate);
+    tc.digest(s);
+    if (k < n_leaves) store_digest(leaves + 8 * k, s);
+  }
+  PICO_TC_CLOSE();
+}
+
 cudaError_t launch_fri_fold_hash_rows(int field, const uint32_t* cw, uint32_t log_len, uint64_t row0,
                                       uint64_t n_leaves, const uint32_t* beta, TwiddleTables tw, uint32_t* out,
                                       uint32_t* leaves, cudaStream_t st) {
   if (n_leaves == 0) return cudaSuccess;
   if (log_len < 2 || 2 * (row0 + 2 * n_leaves) > (1ull << log_len)) return cudaErrorInvalidValue;
+  if (n_leaves >= kTcMinStates)
+    return tc_launch(field == 0 ? k_fri_fold_hash_tc<KoalaBear> : k_fri_fold_hash_tc<BabyBear>, tc_tiles(n_leaves), false,
+                     st, cw, log_len, row0, n_leaves, beta, tw, out, (const uint32_t*)nullptr, leaves);
   if (field == 0)
     k_fri_fold_hash_rows<KoalaBear><<<blocks_for(n_leaves, 256), 256, 0, st>>>(cw, log_len, row0, n_leaves, beta,
                                                                                tw, out, leaves);
@@ -501,6 +831,9 @@ cudaError_t launch_fri_fold_hash(int field, const uint32_t* cw, uint32_t log_len
                                  cudaStream_t st) {
   if (log_len < 2) return cudaErrorInvalidValue;
   const uint64_t n = 1ull << (log_len - 2);
+  if (n >= kTcMinStates)
+    return tc_launch(field == 0 ? k_fri_fold_hash_tc<KoalaBear> : k_fri_fold_hash_tc<BabyBear>, tc_tiles(n), false, st, cw,
+                     log_len, (uint64_t)0, n, beta, tw, out, inject, leaves);
   if (field == 0)
     k_fri_fold_hash<KoalaBear><<<blocks_for(n, 256), 256, 0, st>>>(cw, log_len, beta, tw, out, inject, leaves);
   else

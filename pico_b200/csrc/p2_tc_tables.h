@@ -1,0 +1,53 @@
+// Layout of the tensor-core Poseidon2 tables (p2_tc.cuh), shared by the
+// device code and the host code that builds them (p2_tc_tables.cu).
+#pragma once
+#include <cstdint>
+
+namespace pico {
+
+constexpr uint32_t kTcThreads = 128;  // states per group: M of the MMA, one TMEM lane each
+constexpr uint32_t kTcGroups = 4;      // groups per CTA, sharing the tables
+constexpr uint32_t kTcCtas = 2;        // CTAs per SM
+constexpr uint32_t kTcResident = kTcCtas * 148;  // CTAs of a full wave
+constexpr int kTcBlock = 7;           // partial rounds per block: 7 y words and the constant word fill a 32-byte K step
+constexpr uint32_t kTcCols = 64;      // TMEM columns per group (eight groups fill an SM's 512)
+// TMEM columns of a group: the S-box outputs z of a full round (16 x 64
+// bits) and the accumulators of half a layer (8 words x 4 limbs).
+constexpr uint32_t kTcZ = 0, kTcAcc = 32;
+constexpr int kTcZSteps = 4;
+
+// Shared-memory tables (byte offsets).  A K step is 32 bytes of K for N rows:
+// two core-matrix columns (8 rows x 16 bytes, contiguous) of N / 8 each.
+constexpr uint32_t kTcZero = 0;                      // a zero core-matrix column, N = 64
+constexpr uint32_t kTcFull = 1024;                   // external layer of z: 4 K steps, N = 64
+constexpr uint32_t kTcE2 = kTcFull + 8192;           // external layer of the capacity words of the external layer of z
+constexpr uint32_t kTcNew = kTcE2 + 8192;            // external layer, 8 new rate words: 1 K step
+constexpr uint32_t kTcP1 = kTcNew + 2048;            // first block of partial-round inputs: z, N = 32
+constexpr uint32_t kTcP2 = kTcP1 + 4096;             // second block: z, y_0..6 and the constant (5 steps), N = 32
+constexpr uint32_t kTcP3 = kTcP2 + 5120;             // third block: z, y_0..6, y_7..13 (6 steps), N = 32
+constexpr uint32_t kTcFin = kTcP3 + 6144;            // state after the partial rounds: z and all y (7 steps), N = 64
+constexpr uint32_t kTcC = kTcFin + 14336;            // constant columns, N = 64, 1024 bytes each
+constexpr uint32_t kTcCP1 = kTcC + 9 * 1024;         // constant column of the first block, N = 32
+constexpr uint32_t kTcTableBytes = kTcCP1 + 512;
+// After the tables, the operand words that are not in TMEM, as K steps of 128
+// rows (two core-matrix columns of 2048 bytes): a constant K step whose last
+// word is 1, then per group three of 32-bit words (y of the partial rounds;
+// the rate words to absorb in the second).
+constexpr uint32_t kTcStepBytes = 4096;
+constexpr uint32_t kTcOne = kTcTableBytes;
+constexpr uint32_t kTcY = kTcOne + kTcStepBytes;
+constexpr uint32_t kTcSmemBytes = kTcY + 3 * kTcStepBytes * kTcGroups;
+static_assert(kTcTableBytes % 16 == 0, "operands start on 16 bytes");
+// Indices of the N = 64 constant columns.
+enum TcConstCol : uint32_t { kTcCInit = 0, kTcCMerged = 1, kTcCR1 = 2, kTcCR5 = 5, kTcCOut = 8 };
+
+struct P2TcConstants {
+  int32_t beta[8];  // y of k + 1 rounds ago: Monty form, centred (|.| <= p/2)
+};
+
+// The tables of one field (kTcTableBytes) and its multiply-accumulate
+// constants, from the canonical round constants and diagonal.
+void build_p2_tc_tables(int field, const uint32_t ext[8][16], const uint32_t* inte, const uint32_t diag[16],
+                        uint8_t* tables, P2TcConstants* consts);
+
+}  // namespace pico
