@@ -758,18 +758,15 @@ def run_open(args, rank, world, local):
 # ---------------------------------------------------------------- FRI leg
 def fri_launches(log_n: int, rounds: int, log_final_len: int) -> int:
     """Kernels one commit phase launches (the round loop of fri_host.cu): the
-    first round's leaf hashing; per round the wide compression levels one
-    launch each, seven narrow levels per subtree launch, the tree top with the
+    first round's leaf hashing; per round the levels above 2^14 nodes one launch
+    each, the narrow levels in one (up to 2^7 nodes) or two, the last with the
     challenger step, and the fold (with the next leaves); then the final
     observation (and the final polynomial when it keeps coefficients)."""
     nl = 0
     for r in range(rounds):
-        n = 1 << (log_n - r - 1)
+        log_nodes = log_n - r - 1
         nl += 1 if r == 0 else 0
-        while n > 512:
-            nl += 1
-            n = n >> 7 if n <= (1 << 15) else n // 2
-        nl += 2
+        nl += max(0, log_nodes - 14) + (1 if log_nodes <= 7 else 2) + 1
     return nl + (1 if log_final_len == 0 else 2)
 
 

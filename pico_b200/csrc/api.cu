@@ -737,17 +737,19 @@ pico_status enqueue_tree(const CommitPlan& plan, uint32_t* layers, const std::ve
   uint32_t next_group = 1;
   for (uint32_t lvl = 1; lvl <= log_max;) {
     const uint64_t len = 1ull << (log_max - lvl);  // nodes of the level being made
-    if (2 * len <= (1u << 15) && 2 * len >= kSubtreeIn) {
-      // the narrow levels seven at a time (k_subtree_quad), with the injected
-      // rows of the groups whose heights they meet
+    if (2 * len <= (1u << kSubtreeMaxLog)) {
+      // the narrow levels several at a time (k_subtree_lane), with the
+      // injected rows of the groups whose heights they meet
+      const uint32_t levels = subtree_log_in(log_max - lvl + 1);
       SubtreeInj si{};
-      for (uint32_t l = 0; l < 7; l++)
+      for (uint32_t l = 0; l < levels; l++)
         if (next_group < G && plan.mats[plan.groups[next_group].first].log_N == log_max - (lvl + l))
           si.digests[l] = inj[next_group++];
-      if ((s = cuda_status(launch_subtree(field, layer, (uint32_t)(2 * len), si, st), "compression"))) return s;
+      if ((s = cuda_status(launch_subtree(field, layer, (uint32_t)(2 * len), 1u << levels, si, st), "compression")))
+        return s;
       *launches += 1;
-      for (uint32_t l = 0; l < 7; l++) layer += ((2 * len) >> l) * 8;
-      lvl += 7;
+      for (uint32_t l = 0; l < levels; l++) layer += ((2 * len) >> l) * 8;
+      lvl += levels;
       continue;
     }
     uint32_t* next = layer + (2 * len) * 8;
@@ -1840,8 +1842,8 @@ extern "C" pico_status pico_gpu_autotune(pico_ctx* ctx, pico_field field, uint32
     in_words = std::max<uint64_t>(in_words, (uint64_t)width_for(l) << l);
     out_words = std::max<uint64_t>(out_words, (uint64_t)width_for(l) << (l + 1));
   }
-  // launches of kTcMinStates rows on take no block size
-  const uint64_t hash_rows = kTcMinStates / 2, hash_w = 64;
+  // the launches that take a block size: fewer rows than kTcMinStates, one permutation each
+  const uint64_t hash_rows = kTcMinStates / 2, hash_w = 8;
   out_words = std::max<uint64_t>(out_words, hash_rows * hash_w);
   const uint64_t need = (2 * in_words + 2 * out_words + 2 * kPwWords + hash_rows * 8) * 4;
   if (!try_reserve(ctx, need)) {

@@ -37,30 +37,29 @@ pico_status enqueue_fri_rounds(int field, cudaStream_t st, const TwiddleTables& 
       if ((s = cuda_status(launch_hash_rows(field, g, leaves, trees[0], st), "FRI leaf hashing"))) return s;
       nl++;
     }
-    // wide levels one launch each; from 2^15 nodes down, seven levels per
-    // launch (k_subtree_quad); the last <= 512 nodes and the challenger in
-    // one block
+    // wide levels one launch each; from 2^14 nodes down, the narrow levels in
+    // at most two (k_subtree_lane), the last with the challenger
     uint32_t* layer = trees[r];
-    uint64_t n = leaves;
-    while (n > 512) {
-      if (n <= (1u << 15)) {
-        if ((s = cuda_status(launch_subtree(field, layer, (uint32_t)n, SubtreeInj{}, st), "FRI subtree"))) return s;
-        nl++;
-        for (int l = 0; l < 7; l++) {
-          layer += n * 8;
-          n /= 2;
-        }
-        continue;
-      }
+    uint32_t log_nodes = L - 1;
+    while (log_nodes > kSubtreeMaxLog) {
+      const uint64_t n = 1ull << log_nodes;
       uint32_t* next = layer + n * 8;
       if ((s = cuda_status(launch_compress(field, layer, next, n / 2, nullptr, st), "FRI compression"))) return s;
       nl++;
       layer = next;
-      n /= 2;
+      log_nodes--;
     }
-    if ((s = cuda_status(launch_tree_top(field, layer, (uint32_t)n, d_ch, d_betas + 4 * r, st), "FRI tree top")))
-      return s;
-    nl++;
+    for (bool top = false; !top;) {
+      const uint32_t levels = subtree_log_in(log_nodes);
+      top = levels == log_nodes;
+      if ((s = cuda_status(launch_subtree(field, layer, 1u << log_nodes, 1u << levels, SubtreeInj{}, st,
+                                          top ? d_ch : nullptr, d_betas + 4 * r),
+                           "FRI subtree")))
+        return s;
+      nl++;
+      for (uint32_t l = 0; l < levels; l++) layer += (8ull << log_nodes) >> l;
+      log_nodes -= levels;
+    }
     const uint32_t* inj = inject ? inject[r] : nullptr;
     if (r + 1 < R)
       s = cuda_status(launch_fri_fold_hash(field, codewords[r], L, d_betas + 4 * r, tw, codewords[r + 1], inj,
@@ -311,25 +310,23 @@ pico_status shard_tree_root(pico_fri_shard* fs, uint32_t root[8]) {
   pico_status s;
   const uint64_t leaves = 1ull << (fs->log_rows() - 1);
   uint32_t* layer = fs->tree;
-  uint64_t n = leaves;
-  while (n > 512) {
-    if (n <= (1u << 15)) {
-      if ((s = cuda_status(launch_subtree(fs->field, layer, (uint32_t)n, SubtreeInj{}, fs->st), "FRI subtree")))
-        return s;
-      for (int l = 0; l < 7; l++) {
-        layer += n * 8;
-        n /= 2;
-      }
-      continue;
-    }
+  uint32_t log_nodes = fs->log_rows() - 1;
+  while (log_nodes > kSubtreeMaxLog) {
+    const uint64_t n = 1ull << log_nodes;
     uint32_t* next = layer + n * 8;
     if ((s = cuda_status(launch_compress(fs->field, layer, next, n / 2, nullptr, fs->st), "FRI compression")))
       return s;
     layer = next;
-    n /= 2;
+    log_nodes--;
   }
-  if ((s = cuda_status(launch_tree_top(fs->field, layer, (uint32_t)n, nullptr, nullptr, fs->st), "FRI tree top")))
-    return s;
+  while (log_nodes > 0) {
+    const uint32_t levels = subtree_log_in(log_nodes);
+    if ((s = cuda_status(launch_subtree(fs->field, layer, 1u << log_nodes, 1u << levels, SubtreeInj{}, fs->st),
+                         "FRI subtree")))
+      return s;
+    for (uint32_t l = 0; l < levels; l++) layer += (8ull << log_nodes) >> l;
+    log_nodes -= levels;
+  }
   if ((s = cuda_status(cudaMemcpyAsync(root, fs->tree + (2 * leaves - 2) * 8, 32, cudaMemcpyDeviceToHost, fs->st),
                        "root copy")))
     return s;

@@ -34,8 +34,15 @@ cudaError_t upload_p2_constants(int field, const uint32_t ext[8][16], const uint
 // 2^17 46.2 / 39.1, 2^20 226 / 160.  Below, the latency of one permutation
 // sets the time, and the table load and product stages make it longer.
 constexpr uint64_t kTcMinStates = 1u << 16;
+// Rows of several permutations each: from here on (a row's chain, 2^14 rows of
+// 64 columns: 47 us one thread per row, 38 on the tensor cores).
+constexpr uint64_t kTcMinRows = 1u << 13;
 // four_lanes: four threads per state (the latency form).
 cudaError_t launch_permute(int field, uint32_t* states, uint64_t n, cudaStream_t st, bool four_lanes = false);
+// At most this many states: 16 lanes per state (p2_lane.cuh), bound by latency
+// up to ~2^12 states and by issue above (1.2 G/s against 5 G/s one thread per
+// state); with 2^14 a FRI phase of 2^23 elements took 4.20 instead of 4.11 ms.
+constexpr uint64_t kLaneMaxStates = 8192;
 // Levels of at most this many nodes are compressed four threads per node.
 constexpr uint64_t kQuadMaxNodes = 16384;
 cudaError_t launch_hash_rows(int field, const RowGroup& g, uint64_t rows, uint32_t* out, cudaStream_t st,
@@ -61,13 +68,25 @@ cudaError_t launch_hash_groups(int field, const GroupBatch& b, cudaStream_t st, 
 // the 16-word states to state_out.  Row r's state is 16 consecutive words.
 cudaError_t launch_absorb_rows(int field, const RowGroup& g, uint64_t rows, uint32_t pos0, const uint32_t* state_in,
                                uint32_t* state_out, uint32_t* digest_out, cudaStream_t st, unsigned block = 256);
-// Seven levels at once: a level of n_in nodes (a multiple of 128) down to
-// n_in / 128, every level written after the previous one (tree layout).
-constexpr uint32_t kSubtreeIn = 128;  // input nodes per CTA (seven levels down to one)
+// Levels above a level of n_in nodes, log2 n of them at once, n nodes (a power
+// of two, at most kSubtreeMaxIn) per CTA, every level written after the
+// previous one (tree layout).  With ch (n == n_in): then observe the root and
+// sample beta_out (4 words).
+constexpr uint32_t kSubtreeMaxIn = 128;
 struct SubtreeInj {
   const uint32_t* digests[7];  // per computed level (nullptr: none), 8 words per node
 };
-cudaError_t launch_subtree(int field, uint32_t* level, uint32_t n_in, const SubtreeInj& inj, cudaStream_t st);
+struct DevChallenger;
+cudaError_t launch_subtree(int field, uint32_t* level, uint32_t n_in, uint32_t n, const SubtreeInj& inj,
+                           cudaStream_t st, DevChallenger* ch = nullptr, uint32_t* beta_out = nullptr);
+// The narrow levels of a tree, from 2^log_n <= 2^kSubtreeMaxLog nodes to the
+// root: nodes per CTA (log) of the next launch.  Up to 2^7 nodes go in one
+// launch; above, one over many CTAs leaves 2^6 (from 2^14, 2^7) for another.
+// A level costs its 1.9 us of latency while a CTA has at most 32 nodes to make
+// (two per warp), twice that at 64; a further launch costs about as much as
+// one level.
+constexpr uint32_t kSubtreeMaxLog = 14;
+inline uint32_t subtree_log_in(uint32_t log_n) { return log_n <= 7 ? log_n : log_n <= 13 ? log_n - 6 : 7; }
 // next[i] = compress(prev[2i], prev[2i+1]); if inj_digests != null:
 // next[i] = compress(next[i], inj_digests[i]) (8 words per digest).
 cudaError_t launch_compress(int field, const uint32_t* prev, uint32_t* next, uint64_t n_next,
@@ -136,13 +155,6 @@ cudaError_t launch_fri_fold_hash_rows(int field, const uint32_t* cw, uint32_t lo
 // codeword of 2^log_len EF4 elements; *err set if higher coefficients are nonzero.
 cudaError_t launch_fri_final_poly(int field, const uint32_t* cw, uint32_t log_len, uint32_t log_keep,
                                   TwiddleTables tw, uint32_t* coeffs, uint32_t* err, cudaStream_t st);
-// Observe an 8-element root, then sample 4 elements into beta_out (EF4).
-cudaError_t launch_challenger_round(int field, DevChallenger* ch, const uint32_t* root, uint32_t* beta_out,
-                                    cudaStream_t st);
-// Levels above `level` (n_in <= 512 digests, a power of two) up to the root,
-// written after it; with ch, then observe the root and sample beta_out (4 words).
-cudaError_t launch_tree_top(int field, uint32_t* level, uint32_t n_in, DevChallenger* ch, uint32_t* beta_out,
-                            cudaStream_t st);
 // Observe n elements at vals.
 cudaError_t launch_challenger_observe(int field, DevChallenger* ch, const uint32_t* vals, uint32_t n,
                                       cudaStream_t st);

@@ -10,6 +10,7 @@
 #include "field.cuh"
 #include "internal.h"
 #include "open.h"
+#include "p2_lane.cuh"
 #include "p2_tc.cuh"
 #include "poseidon2.cuh"
 
@@ -26,7 +27,9 @@ cudaError_t upload_p2_constants(int field, const uint32_t ext[8][16], const uint
   if (e) return e;
   std::vector<uint8_t> tables(kTcTableBytes);
   P2TcConstants tc;
-  build_p2_tc_tables(field, h.ext, h.inte, h.diag, tables.data(), &tc);
+  std::vector<uint32_t> lane(kLaneWords);
+  build_p2_tc_tables(field, h.ext, h.inte, h.diag, tables.data(), &tc, lane.data());
+  if ((e = cudaMemcpyToSymbol(g_p2_lane, lane.data(), kLaneWords * 4, (size_t)kLaneWords * 4 * (field ? 1 : 0)))) return e;
   if ((e = cudaMemcpyToSymbol(g_p2_tc, tables.data(), kTcTableBytes, (size_t)kTcTableBytes * (field ? 1 : 0)))) return e;
   return cudaMemcpyToSymbol(c_p2_tc, &tc, sizeof tc, sizeof tc * (field ? 1 : 0));
 }
@@ -249,6 +252,239 @@ __global__ void __launch_bounds__(256)
     p2_permute<F>(s);
   }
   store_digest(next + 8 * i, s);
+}
+
+// ---------------------------------------------------------------------------
+// One word per lane (p2_lane.cuh): 16 lanes per state, for the levels and
+// rows too few to fill the GPU.
+constexpr uint32_t kLaneThreads = 256;  // 16 states per CTA
+
+template <class F>
+__global__ void __launch_bounds__(kLaneThreads) k_compress_lane(const uint32_t* prev, uint32_t* next, uint64_t n,
+                                                                const uint32_t* inj) {
+  __shared__ __align__(16) uint32_t tab[kLaneWords];
+  lane_load_tables<F>(tab);
+  const uint64_t t = blockIdx.x * (uint64_t)kLaneThreads + threadIdx.x;
+  const uint64_t i = t >> 4;
+  const uint32_t q = (uint32_t)(t & 15);
+  const bool live = i < n;
+  uint32_t v = live ? __ldg(prev + 16 * i + q) : 0u;
+  uint32_t d = 0;
+  if (inj && live && q >= 8) d = __ldg(inj + 8 * i + q - 8);
+  __syncthreads();
+  v = lane_permute<F>(v, q, tab);
+  if (inj) {
+    if (q >= 8) v = d;
+    v = lane_permute<F>(v, q, tab);
+  }
+  if (live && q < 8) next[8 * i + q] = v;
+}
+
+// Row digests of a GroupBatch, 16 lanes per row (k_hash_groups' sponges): lanes
+// 0..7 carry the rate, so a chunk's eight words are one load.
+template <class F>
+__global__ void __launch_bounds__(kLaneThreads) k_hash_groups_lane(const __grid_constant__ GroupBatch b) {
+  __shared__ __align__(16) uint32_t tab[kLaneWords];
+  lane_load_tables<F>(tab);
+  __syncthreads();
+  if (b.n_groups == 0 || b.n_groups > (uint32_t)kBatchGroups) return;
+  const uint64_t t = blockIdx.x * (uint64_t)kLaneThreads + threadIdx.x;
+  const uint64_t row = t >> 4;
+  const uint32_t q = (uint32_t)(t & 15);
+  const bool live = row < b.row_end[b.n_groups - 1];
+  uint32_t g = 0;
+  while (g + 1 < b.n_groups && row >= b.row_end[g]) g++;
+  const uint64_t r = row - (g ? b.row_end[g - 1] : 0ull);
+  const uint32_t s0 = b.seg_begin[g], s1 = b.seg_begin[g + 1];
+  uint32_t W = live ? b.width[g] : 0u;
+  if (s1 < s0 || s1 > (uint32_t)kBatchSegs) {
+    hash_guard_trip(s0, s1);
+    W = 0;
+  }
+  // the two rows of a warp may differ in width: the warp runs the longer one's
+  // chunks, the other keeps its digest
+  const uint32_t chunks = (W + 7) / 8;
+  const uint32_t steps = max(chunks, __shfl_xor_sync(0xffffffffu, chunks, 16));
+  uint32_t seg = s0, begin = 0;  // this lane's segment and its first column
+  uint32_t v = 0;
+  for (uint32_t c = 0; c < steps; c++) {
+    const uint32_t col = 8 * c + q;
+    uint32_t w = v;
+    if (q < 8 && col < W) {
+      while (seg < s1 && col - begin >= b.segs[seg].width) begin += b.segs[seg++].width;
+      if (seg >= s1) {
+        hash_guard_trip(seg, col);
+        w = 0;
+      } else {
+        w = __ldg(b.segs[seg].ptr + r * b.segs[seg].width + (col - begin));
+      }
+    }
+    w = lane_permute<F>(w, q, tab);
+    if (c < chunks) v = w;
+  }
+  if (live && q < 8) b.out[g][8 * r + q] = v;
+}
+
+// k_absorb_rows with 16 lanes per row.
+template <class F>
+__global__ void __launch_bounds__(kLaneThreads)
+    k_absorb_rows_lane(const __grid_constant__ RowGroup g, uint64_t rows, uint32_t pos0, const uint32_t* state_in,
+                       uint32_t* state_out, uint32_t* digest_out) {
+  __shared__ __align__(16) uint32_t tab[kLaneWords];
+  lane_load_tables<F>(tab);
+  __syncthreads();
+  const uint64_t t = blockIdx.x * (uint64_t)kLaneThreads + threadIdx.x;
+  const uint64_t r = t >> 4;
+  const uint32_t q = (uint32_t)(t & 15);
+  const bool live = r < rows;
+  uint32_t v = live && state_in ? state_in[16 * r + q] : 0u;
+  const uint32_t end = pos0 + g.total_width;
+  uint32_t seg = 0, begin = 0;  // this lane's segment and its first column
+  for (uint32_t base = 0; base < end; base += 8) {
+    const uint32_t c = base + q;  // chunk position; column c - pos0 of this call
+    if (live && q < 8 && c >= pos0 && c < end) {
+      const uint32_t col = c - pos0;
+      while (seg < g.n_segs && col - begin >= g.segs[seg].width) begin += g.segs[seg++].width;
+      if (seg >= g.n_segs) {
+        hash_guard_trip(seg, col);
+        v = 0;
+      } else {
+        v = __ldg(g.segs[seg].ptr + r * g.segs[seg].width + (col - begin));
+      }
+    }
+    if (base + 8 <= end || digest_out) v = lane_permute<F>(v, q, tab);
+  }
+  if (!live) return;
+  if (!digest_out)
+    state_out[16 * r + q] = v;
+  else if (q < 8)
+    digest_out[8 * r + q] = v;
+}
+
+// Duplex challenger (challenger.rs:89-115, 202-237) held by the 16 lanes of a
+// warp's halves: lane q has sponge word q and buffer words q mod 8.
+template <class F>
+struct LaneChallenger {
+  uint32_t sponge, in, out, in_len, out_len;
+  __device__ __forceinline__ void load(const DevChallenger* ch, uint32_t q) {
+    sponge = ch->sponge[q];
+    in = ch->in_buf[q & 7];
+    out = ch->out_buf[q & 7];
+    in_len = ch->in_len;
+    out_len = ch->out_len;
+  }
+  __device__ __forceinline__ void store(DevChallenger* ch, uint32_t q) const {
+    ch->sponge[q] = sponge;
+    if (q < 8) {
+      ch->in_buf[q] = in;
+      ch->out_buf[q] = out;
+    }
+    if (q == 0) {
+      ch->in_len = in_len;
+      ch->out_len = out_len;
+    }
+  }
+  __device__ __forceinline__ void duplex(uint32_t q, const uint32_t* tab) {
+    sponge = lane_permute<F>(q < in_len ? in : sponge, q, tab);
+    in_len = 0;
+    out = __shfl_sync(0xffffffffu, sponge, (int)(q & 7), 16);
+    out_len = 8;
+  }
+  __device__ __forceinline__ void observe(uint32_t value, uint32_t q, const uint32_t* tab) {
+    out_len = 0;
+    if ((q & 7) == in_len) in = value;
+    if (++in_len == 8) duplex(q, tab);
+  }
+  __device__ __forceinline__ uint32_t sample(uint32_t q, const uint32_t* tab) {
+    if (in_len != 0 || out_len == 0) duplex(q, tab);
+    return __shfl_sync(0xffffffffu, out, (int)--out_len, 16);
+  }
+};
+
+// Levels of a tree above `n` nodes (a power of two), in one CTA, in shared
+// memory: cur holds the nodes, spare is as large as half of them; every level is written
+// after the previous one (in the whole tree the level holds total nodes, this
+// CTA's are those from c * n).  Returns the buffer that holds the last node.
+constexpr uint32_t kSubtreeThreads = 512;
+template <class F>
+__device__ __forceinline__ uint32_t* lane_subtree(uint32_t* cur, uint32_t* spare, uint32_t n, uint32_t* level,
+                                                  uint64_t total, uint64_t c, const SubtreeInj* inj,
+                                                  const uint32_t* tab) {
+  const uint32_t q = threadIdx.x & 15, g = threadIdx.x >> 4;
+  uint32_t lvl = 0;
+  while (n > 1) {
+    const uint32_t m = n >> 1;
+    uint32_t* out = level + 8 * total;
+    const uint32_t* d = inj ? inj->digests[lvl] : nullptr;
+    for (uint32_t s = 0; s < m; s += kSubtreeThreads / 16) {
+      if (s + (threadIdx.x >> 5) * 2 >= m) break;  // warp-uniform
+      const uint32_t node = s + g;
+      const bool live = node < m;
+      uint32_t v = live ? cur[16 * node + q] : 0u;
+      uint32_t w = 0;
+      if (d && live && q >= 8) w = __ldg(d + (c * m + node) * 8 + q - 8);
+      v = lane_permute<F>(v, q, tab);
+      if (d) {
+        if (q >= 8) v = w;
+        v = lane_permute<F>(v, q, tab);
+      }
+      if (live && q < 8) {
+        spare[8 * node + q] = v;
+        out[(c * m + node) * 8 + q] = v;
+      }
+    }
+    __syncthreads();
+    uint32_t* t = cur;
+    cur = spare;
+    spare = t;
+    level = out;
+    total >>= 1;
+    n = m;
+    lvl++;
+  }
+  return cur;
+}
+
+// The levels above CTA c's nodes [c * n, (c + 1) * n) of a level of n_in nodes;
+// with a challenger (one CTA only), then observe the root and sample the EF4
+// challenge into beta_out.
+template <class F>
+__global__ void __launch_bounds__(kSubtreeThreads)
+    k_subtree_lane(uint32_t* level, uint32_t n_in, uint32_t n, const __grid_constant__ SubtreeInj inj,
+                   DevChallenger* ch, uint32_t* beta_out) {
+  __shared__ __align__(16) uint32_t tab[kLaneWords];
+  __shared__ __align__(16) uint32_t buf[(kSubtreeMaxIn + kSubtreeMaxIn / 2) * 8];
+  lane_load_tables<F>(tab);
+  if (n > kSubtreeMaxIn || (uint64_t)(blockIdx.x + 1) * n > n_in) return;  // the launcher checks both
+  const uint32_t* src = level + (size_t)blockIdx.x * n * 8;
+  for (uint32_t i = threadIdx.x; i < n * 8; i += kSubtreeThreads) buf[i] = src[i];
+  __syncthreads();
+  const uint32_t* root = lane_subtree<F>(buf, buf + kSubtreeMaxIn * 8, n, level, n_in, blockIdx.x, &inj, tab);
+  if (ch && threadIdx.x < 32) {
+    const uint32_t q = threadIdx.x & 15;
+    LaneChallenger<F> c;
+    c.load(ch, q);
+    for (int i = 0; i < 8; i++) c.observe(root[i], q, tab);
+    uint32_t beta = 0;
+    for (uint32_t i = 0; i < 4; i++) {
+      const uint32_t b = c.sample(q, tab);
+      if (q == i) beta = b;
+    }
+    if (threadIdx.x < 4) beta_out[threadIdx.x] = beta;
+    if (threadIdx.x < 16) c.store(ch, q);
+  }
+}
+
+template <class F>
+__global__ void k_challenger_observe(DevChallenger* ch, const uint32_t* vals, uint32_t n) {
+  __shared__ __align__(16) uint32_t tab[kLaneWords];
+  lane_load_tables<F>(tab);
+  __syncthreads();
+  const uint32_t q = threadIdx.x & 15;
+  LaneChallenger<F> c;
+  c.load(ch, q);
+  for (uint32_t i = 0; i < n; i++) c.observe(vals[i], q, tab);
+  if (threadIdx.x < 16) c.store(ch, q);
 }
 
 // ---------------------------------------------------------------------------
@@ -546,22 +782,32 @@ cudaError_t hash_guard_clear() {
   return cudaMemcpyToSymbol(g_hash_guard, &z, sizeof z);
 }
 
-// block: threads per CTA, 32 .. 256 (the kernels are bounded to 256).
+// Rows are hashed on the tensor cores when there are enough states for one
+// permutation, or, where each takes several, from kTcMinRows on.
+static bool use_tensor_rows(uint64_t rows, uint64_t chunks) {
+  return rows >= kTcMinStates || (rows >= kTcMinRows && chunks >= 2);
+}
+// A batch of one group.
+static GroupBatch one_group(const RowGroup& g, uint64_t rows, uint32_t* out) {
+  GroupBatch b;
+  memset(&b, 0, sizeof b);
+  b.n_groups = 1;
+  b.n_segs = g.n_segs;
+  b.row_end[0] = rows;
+  b.out[0] = out;
+  b.seg_begin[1] = g.n_segs;
+  b.width[0] = g.total_width;
+  for (uint32_t k = 0; k < g.n_segs; k++) b.segs[k] = g.segs[k];
+  return b;
+}
+
+// block: threads per CTA, 32 .. 256 (the kernels are bounded to 256), where
+// rows are hashed one thread each.
 cudaError_t launch_hash_rows(int field, const RowGroup& g, uint64_t rows, uint32_t* out, cudaStream_t st,
                              unsigned block) {
   if (rows == 0) return cudaSuccess;
-  if (rows >= kTcMinStates) {
-    GroupBatch b;
-    memset(&b, 0, sizeof b);
-    b.n_groups = 1;
-    b.n_segs = g.n_segs;
-    b.row_end[0] = rows;
-    b.out[0] = out;
-    b.seg_begin[1] = g.n_segs;
-    b.width[0] = g.total_width;
-    for (uint32_t k = 0; k < g.n_segs; k++) b.segs[k] = g.segs[k];
-    return launch_hash_groups(field, b, st, block);
-  }
+  if (use_tensor_rows(rows, (g.total_width + 7) / 8) || rows <= kLaneMaxStates)
+    return launch_hash_groups(field, one_group(g, rows, out), st, block);
   if (block < 32 || block > 256) block = 256;
   if (field == 0)
     k_hash_rows<KoalaBear><<<blocks_for(rows, block), block, 0, st>>>(g, rows, out);
@@ -575,15 +821,22 @@ cudaError_t launch_hash_groups(int field, const GroupBatch& b, cudaStream_t st, 
   if (b.n_groups > (uint32_t)kBatchGroups || b.n_segs > (uint32_t)kBatchSegs) return cudaErrorInvalidValue;
   const uint64_t rows = b.row_end[b.n_groups - 1];
   if (rows == 0) return cudaSuccess;
-  if (rows >= kTcMinStates) {
-    uint64_t tiles = 0, chunks = 0;
-    for (uint32_t g = 0; g < b.n_groups; g++) {
-      const uint64_t t = tc_tiles(b.row_end[g] - (g ? b.row_end[g - 1] : 0ull));
-      tiles += t;
-      chunks += t * ((b.width[g] + 7) / 8);
-    }
+  uint64_t tiles = 0, chunks = 0;
+  for (uint32_t g = 0; g < b.n_groups; g++) {
+    const uint64_t t = tc_tiles(b.row_end[g] - (g ? b.row_end[g - 1] : 0ull));
+    tiles += t;
+    chunks += t * ((b.width[g] + 7) / 8);
+  }
+  if (use_tensor_rows(rows, chunks / tiles)) {
     return tc_launch(field == 0 ? k_hash_groups_tc<KoalaBear> : k_hash_groups_tc<BabyBear>, tiles,
                      chunks >= kTcWholeChunks * tiles, st, b, tiles);
+  }
+  if (rows <= kLaneMaxStates) {
+    if (field == 0)
+      k_hash_groups_lane<KoalaBear><<<blocks_for(16 * rows, kLaneThreads), kLaneThreads, 0, st>>>(b);
+    else
+      k_hash_groups_lane<BabyBear><<<blocks_for(16 * rows, kLaneThreads), kLaneThreads, 0, st>>>(b);
+    return cudaGetLastError();
   }
   if (block < 32 || block > 256) block = 256;
   if (field == 0)
@@ -596,9 +849,19 @@ cudaError_t launch_hash_groups(int field, const GroupBatch& b, cudaStream_t st, 
 cudaError_t launch_absorb_rows(int field, const RowGroup& g, uint64_t rows, uint32_t pos0, const uint32_t* state_in,
                                uint32_t* state_out, uint32_t* digest_out, cudaStream_t st, unsigned block) {
   if (rows == 0) return cudaSuccess;
-  if (rows >= kTcMinStates) {
-    return tc_launch(field == 0 ? k_absorb_rows_tc<KoalaBear> : k_absorb_rows_tc<BabyBear>, tc_tiles(rows), pos0 + g.total_width >= 8 * kTcWholeChunks, st,
+  const uint64_t absorbed = pos0 + g.total_width;
+  if (use_tensor_rows(rows, absorbed / 8)) {
+    return tc_launch(field == 0 ? k_absorb_rows_tc<KoalaBear> : k_absorb_rows_tc<BabyBear>, tc_tiles(rows), absorbed >= 8 * kTcWholeChunks, st,
                      g, rows, pos0, state_in, state_out, digest_out);
+  }
+  if (rows <= kLaneMaxStates) {
+    if (field == 0)
+      k_absorb_rows_lane<KoalaBear><<<blocks_for(16 * rows, kLaneThreads), kLaneThreads, 0, st>>>(
+          g, rows, pos0, state_in, state_out, digest_out);
+    else
+      k_absorb_rows_lane<BabyBear><<<blocks_for(16 * rows, kLaneThreads), kLaneThreads, 0, st>>>(
+          g, rows, pos0, state_in, state_out, digest_out);
+    return cudaGetLastError();
   }
   if (block < 32 || block > 256) block = 256;
   if (field == 0)
@@ -643,6 +906,13 @@ __global__ void __launch_bounds__(256) k_compress_quad(const uint32_t* prev, uin
 cudaError_t launch_compress(int field, const uint32_t* prev, uint32_t* next, uint64_t n_next,
                             const uint32_t* inj_digests, cudaStream_t st) {
   if (n_next == 0) return cudaSuccess;
+  if (n_next <= kLaneMaxStates) {
+    if (field == 0)
+      k_compress_lane<KoalaBear><<<blocks_for(16 * n_next, kLaneThreads), kLaneThreads, 0, st>>>(prev, next, n_next, inj_digests);
+    else
+      k_compress_lane<BabyBear><<<blocks_for(16 * n_next, kLaneThreads), kLaneThreads, 0, st>>>(prev, next, n_next, inj_digests);
+    return cudaGetLastError();
+  }
   if (n_next <= kQuadMaxNodes) {
     if (field == 0)
       k_compress_quad<KoalaBear><<<blocks_for(4 * n_next, 256), 256, 0, st>>>(prev, next, n_next, inj_digests);
@@ -772,6 +1042,32 @@ __global__ void __launch_bounds__(256) k_fri_fold_hash_rows(const uint32_t* cw, 
   lp[1] = make_uint4(s[4], s[5], s[6], s[7]);
 }
 
+// The same with 16 lanes per leaf (p2_lane.cuh): lane q < 8 folds the row of
+// the leaf's word q (every lane of a row computes the whole element).
+template <class F>
+__global__ void __launch_bounds__(kLaneThreads)
+    k_fri_fold_hash_lane(const uint32_t* cw, uint32_t log_len, uint64_t row0, uint64_t n_leaves, const uint32_t* beta,
+                         const __grid_constant__ TwiddleTables tw, uint32_t* out, const uint32_t* inject,
+                         uint32_t* leaves) {
+  __shared__ __align__(16) uint32_t tab[kLaneWords];
+  lane_load_tables<F>(tab);
+  const uint64_t t = blockIdx.x * (uint64_t)kLaneThreads + threadIdx.x;
+  const uint64_t k = t >> 4;
+  const uint32_t q = (uint32_t)(t & 15);
+  const bool live = k < n_leaves;
+  uint32_t v = 0;
+  if (live && q < 8) {
+    const uint64_t r = 2 * k + (q >> 2);
+    const Ext4 res = fri_fold_row<F>(cw, log_len, r, half_beta<F>(beta), tw, row0 + r);
+    v = (q & 2) ? ((q & 1) ? res.c[3] : res.c[2]) : ((q & 1) ? res.c[1] : res.c[0]);
+    if (inject) v = Fp<F>::add(v, __ldg(inject + 4 * r + (q & 3)));
+    out[4 * r + (q & 3)] = v;
+  }
+  __syncthreads();
+  v = lane_permute<F>(v, q, tab);
+  if (live && q < 8) leaves[8 * k + q] = v;
+}
+
 // k_fri_fold_hash and k_fri_fold_hash_rows with the leaves hashed on the
 // tensor cores (p2_tc.cuh).
 template <class F>
@@ -809,6 +1105,18 @@ __global__ void __launch_bounds__(kTcThreads * kTcGroups, kTcCtas)
   PICO_TC_CLOSE();
 }
 
+static cudaError_t launch_fri_fold_hash_lane(int field, const uint32_t* cw, uint32_t log_len, uint64_t row0, uint64_t n,
+                                             const uint32_t* beta, TwiddleTables tw, uint32_t* out,
+                                             const uint32_t* inject, uint32_t* leaves, cudaStream_t st) {
+  if (field == 0)
+    k_fri_fold_hash_lane<KoalaBear><<<blocks_for(16 * n, kLaneThreads), kLaneThreads, 0, st>>>(cw, log_len, row0, n, beta,
+                                                                                              tw, out, inject, leaves);
+  else
+    k_fri_fold_hash_lane<BabyBear><<<blocks_for(16 * n, kLaneThreads), kLaneThreads, 0, st>>>(cw, log_len, row0, n, beta,
+                                                                                             tw, out, inject, leaves);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_fri_fold_hash_rows(int field, const uint32_t* cw, uint32_t log_len, uint64_t row0,
                                       uint64_t n_leaves, const uint32_t* beta, TwiddleTables tw, uint32_t* out,
                                       uint32_t* leaves, cudaStream_t st) {
@@ -817,6 +1125,8 @@ cudaError_t launch_fri_fold_hash_rows(int field, const uint32_t* cw, uint32_t lo
   if (n_leaves >= kTcMinStates)
     return tc_launch(field == 0 ? k_fri_fold_hash_tc<KoalaBear> : k_fri_fold_hash_tc<BabyBear>, tc_tiles(n_leaves), false,
                      st, cw, log_len, row0, n_leaves, beta, tw, out, (const uint32_t*)nullptr, leaves);
+  if (n_leaves <= kLaneMaxStates)
+    return launch_fri_fold_hash_lane(field, cw, log_len, row0, n_leaves, beta, tw, out, nullptr, leaves, st);
   if (field == 0)
     k_fri_fold_hash_rows<KoalaBear><<<blocks_for(n_leaves, 256), 256, 0, st>>>(cw, log_len, row0, n_leaves, beta,
                                                                                tw, out, leaves);
@@ -834,6 +1144,8 @@ cudaError_t launch_fri_fold_hash(int field, const uint32_t* cw, uint32_t log_len
   if (n >= kTcMinStates)
     return tc_launch(field == 0 ? k_fri_fold_hash_tc<KoalaBear> : k_fri_fold_hash_tc<BabyBear>, tc_tiles(n), false, st, cw,
                      log_len, (uint64_t)0, n, beta, tw, out, inject, leaves);
+  if (n <= kLaneMaxStates)
+    return launch_fri_fold_hash_lane(field, cw, log_len, 0, n, beta, tw, out, inject, leaves, st);
   if (field == 0)
     k_fri_fold_hash<KoalaBear><<<blocks_for(n, 256), 256, 0, st>>>(cw, log_len, beta, tw, out, inject, leaves);
   else
@@ -851,191 +1163,13 @@ cudaError_t launch_fri_fold_tw(int field, const uint32_t* cw, uint32_t log_len, 
   return cudaGetLastError();
 }
 
-// Duplex challenger (challenger.rs:89-115, 202-237), one thread.
-template <class F>
-__device__ void ch_duplex(DevChallenger* ch) {
-  uint32_t s[16];
-  for (int i = 0; i < 16; i++) s[i] = ch->sponge[i];
-  for (uint32_t i = 0; i < ch->in_len; i++) s[i] = ch->in_buf[i];
-  ch->in_len = 0;
-  p2_permute<F>(s);
-  for (int i = 0; i < 16; i++) ch->sponge[i] = s[i];
-  for (int i = 0; i < 8; i++) ch->out_buf[i] = s[i];
-  ch->out_len = 8;
-}
-
-template <class F>
-__device__ void ch_observe(DevChallenger* ch, uint32_t v) {
-  ch->out_len = 0;
-  ch->in_buf[ch->in_len++] = v;
-  if (ch->in_len == 8) ch_duplex<F>(ch);
-}
-
-template <class F>
-__device__ uint32_t ch_sample(DevChallenger* ch) {
-  if (ch->in_len != 0 || ch->out_len == 0) ch_duplex<F>(ch);
-  return ch->out_buf[--ch->out_len];
-}
-
-template <class F>
-__global__ void k_challenger_round(DevChallenger* ch, const uint32_t* root, uint32_t* beta_out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  for (int i = 0; i < 8; i++) ch_observe<F>(ch, root[i]);
-  for (int i = 0; i < 4; i++) beta_out[i] = ch_sample<F>(ch);
-}
-
-template <class F>
-__global__ void k_challenger_observe(DevChallenger* ch, const uint32_t* vals, uint32_t n) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  for (uint32_t i = 0; i < n; i++) ch_observe<F>(ch, vals[i]);
-}
-
-// The top of a Merkle tree in one block: `level` holds n_in <= 512 digests
-// (a power of two); every level above it is computed in shared memory and
-// written after it (the layer layout: each level follows the one below), up
-// to the root.  With a challenger, thread 0 then observes the root and samples
-// the EF4 challenge into beta_out (k_challenger_round's step).
-constexpr uint32_t kTreeTopMax = 512;
-
-template <class F>
-__global__ void __launch_bounds__(256) k_tree_top(uint32_t* level, uint32_t n_in, DevChallenger* ch,
-                                                  uint32_t* beta_out) {
-  __shared__ uint32_t buf[kTreeTopMax * 8];
-  const uint32_t tid = threadIdx.x;
-  for (uint32_t i = tid; i < n_in * 8; i += blockDim.x) buf[i] = level[i];
-  __syncthreads();
-  uint32_t n = n_in;
-  uint32_t* in = level;
-  while (n > 1) {
-    const uint32_t m = n >> 1;
-    uint32_t* out = in + (size_t)n * 8;
-    if (m > 64) {
-      // one thread per node
-      uint32_t st[16];
-      if (tid < m) {
-#pragma unroll
-        for (int k = 0; k < 16; k++) st[k] = buf[16 * tid + k];
-        p2_permute<F>(st);
-      }
-      __syncthreads();
-      if (tid < m) {
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-          buf[8 * tid + k] = st[k];
-          out[8 * tid + k] = st[k];
-        }
-      }
-    } else {
-      // four threads per node (4m <= 256): the latency form
-      const uint32_t node = tid >> 2, q = tid & 3;
-      uint32_t v[4];
-      if (tid < 4 * m) {
-        const unsigned mask = 4 * m >= 32 ? 0xffffffffu : ((1u << (4 * m)) - 1u);
-#pragma unroll
-        for (int k = 0; k < 4; k++) v[k] = buf[16 * node + 4 * q + k];
-        p2_permute_quad<F>(v, q, mask);
-      }
-      __syncthreads();
-      if (tid < 4 * m && q < 2) {
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-          buf[8 * node + 4 * q + k] = v[k];
-          out[8 * node + 4 * q + k] = v[k];
-        }
-      }
-    }
-    __syncthreads();
-    in = out;
-    n = m;
-  }
-  if (ch && tid == 0) {
-    for (int i = 0; i < 8; i++) ch_observe<F>(ch, buf[i]);
-    for (int i = 0; i < 4; i++) beta_out[i] = ch_sample<F>(ch);
-  }
-}
-
-// Seven compression levels in one launch: CTA c reduces input nodes
-// [128 c, 128 c + 128) of a level of n_in nodes to one node, four lanes per
-// state, and writes every level it computes to the tree (level l + 1 follows
-// level l, which holds n_in >> l nodes).  n_in is a multiple of 128.  Where
-// inj.digests[l] is set, node i of computed level l is compressed once more
-// with digest i of it (a commit's injected rows).  For the narrow levels of a
-// tree this replaces seven latency-bound launches.
-template <class F>
-__global__ void __launch_bounds__(256) k_subtree_quad(uint32_t* level, uint32_t n_in,
-                                                      const __grid_constant__ SubtreeInj inj) {
-  __shared__ uint32_t buf[kSubtreeIn * 8];
-  const uint32_t tid = threadIdx.x, c = blockIdx.x;
-  if ((uint64_t)(c + 1) * kSubtreeIn > n_in) return;  // whole chunks only (the launcher checks n_in)
-  const uint32_t* src = level + (size_t)c * kSubtreeIn * 8;
-  for (uint32_t i = tid; i < kSubtreeIn * 8; i += blockDim.x) buf[i] = src[i];
-  __syncthreads();
-  uint32_t n = kSubtreeIn;  // this CTA's nodes at the current level
-  uint32_t nl = n_in;       // the whole level's nodes
-  uint32_t* in = level;
-  uint32_t lvl = 0;         // levels computed so far
-  while (n > 1) {
-    const uint32_t m = n >> 1;
-    uint32_t* out = in + (size_t)nl * 8;
-    const uint32_t node = tid >> 2, q = tid & 3;
-    const bool live = tid < 4 * m;
-    uint32_t v[4];
-    const uint32_t* d = inj.digests[lvl];
-    if (live) {
-      const unsigned mask = 4 * m >= 32 ? 0xffffffffu : ((1u << (4 * m)) - 1u);
-#pragma unroll
-      for (int k = 0; k < 4; k++) v[k] = buf[16 * node + 4 * q + k];
-      p2_permute_quad<F>(v, q, mask);
-      if (d) {
-        // compress(node, injected digest): lanes 2, 3 load the injection
-        if (q >= 2) {
-          const uint4 a = __ldg(reinterpret_cast<const uint4*>(d + ((size_t)c * m + node) * 8) + (q - 2));
-          v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-        }
-        p2_permute_quad<F>(v, q, mask);
-      }
-    }
-    __syncthreads();
-    if (live && q < 2) {
-#pragma unroll
-      for (int k = 0; k < 4; k++) {
-        buf[8 * node + 4 * q + k] = v[k];
-        out[((size_t)c * m + node) * 8 + 4 * q + k] = v[k];
-      }
-    }
-    __syncthreads();
-    in = out;
-    nl >>= 1;
-    n = m;
-    lvl++;
-  }
-}
-
-cudaError_t launch_subtree(int field, uint32_t* level, uint32_t n_in, const SubtreeInj& inj, cudaStream_t st) {
-  if (n_in < kSubtreeIn || n_in % kSubtreeIn) return cudaErrorInvalidValue;
+cudaError_t launch_subtree(int field, uint32_t* level, uint32_t n_in, uint32_t n, const SubtreeInj& inj,
+                           cudaStream_t st, DevChallenger* ch, uint32_t* beta_out) {
+  if (n == 0 || n > kSubtreeMaxIn || (n & (n - 1)) || n_in % n || (ch && n != n_in)) return cudaErrorInvalidValue;
   if (field == 0)
-    k_subtree_quad<KoalaBear><<<n_in / kSubtreeIn, 256, 0, st>>>(level, n_in, inj);
+    k_subtree_lane<KoalaBear><<<n_in / n, kSubtreeThreads, 0, st>>>(level, n_in, n, inj, ch, beta_out);
   else
-    k_subtree_quad<BabyBear><<<n_in / kSubtreeIn, 256, 0, st>>>(level, n_in, inj);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_tree_top(int field, uint32_t* level, uint32_t n_in, DevChallenger* ch, uint32_t* beta_out,
-                            cudaStream_t st) {
-  if (n_in == 0 || n_in > kTreeTopMax || (n_in & (n_in - 1))) return cudaErrorInvalidValue;
-  if (field == 0)
-    k_tree_top<KoalaBear><<<1, 256, 0, st>>>(level, n_in, ch, beta_out);
-  else
-    k_tree_top<BabyBear><<<1, 256, 0, st>>>(level, n_in, ch, beta_out);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_challenger_round(int field, DevChallenger* ch, const uint32_t* root, uint32_t* beta_out,
-                                    cudaStream_t st) {
-  if (field == 0)
-    k_challenger_round<KoalaBear><<<1, 32, 0, st>>>(ch, root, beta_out);
-  else
-    k_challenger_round<BabyBear><<<1, 32, 0, st>>>(ch, root, beta_out);
+    k_subtree_lane<BabyBear><<<n_in / n, kSubtreeThreads, 0, st>>>(level, n_in, n, inj, ch, beta_out);
   return cudaGetLastError();
 }
 

@@ -59,7 +59,7 @@ struct Builder {
 
 template <class F>
 void build(const uint32_t ext[8][16], const uint32_t* inte, const uint32_t diag[16], uint8_t* tables,
-           P2TcConstants* consts) {
+           P2TcConstants* consts, uint32_t* lane) {
   constexpr int R = F::ROUNDS_P;
   Builder B;
   B.p = F::P;
@@ -175,16 +175,33 @@ void build(const uint32_t ext[8][16], const uint32_t* inte, const uint32_t diag[
     const uint64_t v = (B.mul(ext[4][i], S) + 2 * p - B.mul(B.mul(sum, S), off) - B.mul(B.mul(sum_z, SZ), off_z)) % p;
     B.constant_step(kTcFin + 2048 * kTcZSteps, 64, i, v);
   }
+
+  // the one-word-per-lane tables: canonical values in Monty form
+  memset(lane, 0, kLaneWords * 4);
+  auto monty = [&](uint64_t v) { return (uint32_t)B.mul(v, B.r32); };
+  for (uint32_t i = 0; i < 16; i++) {
+    for (uint32_t r = 0; r < 8; r++) lane[kLaneExt + 16 * r + i] = ext[r][i];
+    for (uint32_t j = 0; j < 16; j++) {
+      if ((int)i < R) lane[kLaneAlpha + 16 * j + i] = monty(alpha[i][j]);
+      if ((int)(16 + i) < R) lane[kLaneAlpha + 256 + 16 * j + i] = monty(alpha[16 + i][j]);
+      lane[kLaneGamma + 16 * j + i] = monty(gamma[i][j]);
+    }
+    for (int t = 0; t < R; t++) lane[kLaneG + 16 * t + i] = monty(g[R - 1 - t][i]);
+    if ((int)i < R) lane[kLaneConst + i] = monty(inte[i]);
+    if ((int)(16 + i) < R) lane[kLaneConst + 16 + i] = monty(inte[16 + i]);
+    lane[kLaneConst + 32 + i] = monty(ext[4][i]);
+  }
+  for (int k = 0; k < R; k++) lane[kLaneBeta + kLaneBetaZero + k] = monty(beta[k]);
 }
 
 }  // namespace
 
 void build_p2_tc_tables(int field, const uint32_t ext[8][16], const uint32_t* inte, const uint32_t diag[16],
-                        uint8_t* tables, P2TcConstants* consts) {
+                        uint8_t* tables, P2TcConstants* consts, uint32_t* lane) {
   if (field == 0)
-    build<KoalaBear>(ext, inte, diag, tables, consts);
+    build<KoalaBear>(ext, inte, diag, tables, consts, lane);
   else
-    build<BabyBear>(ext, inte, diag, tables, consts);
+    build<BabyBear>(ext, inte, diag, tables, consts, lane);
 }
 
 }  // namespace pico

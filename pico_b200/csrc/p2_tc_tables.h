@@ -45,9 +45,21 @@ struct P2TcConstants {
   int32_t beta[8];  // y of k + 1 rounds ago: Monty form, centred (|.| <= p/2)
 };
 
+// Tables of the one-word-per-lane form (p2_lane.cuh), in words; entry [k][i]
+// belongs to lane i.
+constexpr uint32_t kLaneExt = 0;                      // full-round constants, 8 x 16
+constexpr uint32_t kLaneAlpha = 128;                  // alpha_i per z_j, 16 x 16, then alpha_(16+i)
+constexpr uint32_t kLaneGamma = kLaneAlpha + 512;     // Gamma, 16 x 16
+constexpr uint32_t kLaneG = kLaneGamma + 256;         // state after the partial rounds per y_t, 20 x 16
+constexpr uint32_t kLaneConst = kLaneG + 320;         // c_i, c_(16+i), constants of the next full round, times 2^32
+constexpr uint32_t kLaneBeta = kLaneConst + 48;       // beta_k at kLaneBetaZero + k, zero elsewhere
+constexpr uint32_t kLaneBetaZero = 24;
+constexpr uint32_t kLaneWords = kLaneBeta + 64;
+static_assert(kLaneWords % 4 == 0, "copied by 16 bytes");
+
 // The tables of one field (kTcTableBytes) and its multiply-accumulate
-// constants, from the canonical round constants and diagonal.
+// constants, and the lane tables (kLaneWords), from the canonical round constants and diagonal.
 void build_p2_tc_tables(int field, const uint32_t ext[8][16], const uint32_t* inte, const uint32_t diag[16],
-                        uint8_t* tables, P2TcConstants* consts);
+                        uint8_t* tables, P2TcConstants* consts, uint32_t* lane);
 
 }  // namespace pico
