@@ -1079,6 +1079,11 @@ struct HashBatcher {
   }
 };
 
+// Commits of at most this many trace cells launch all their LDEs together;
+// above, the tallest group's runs just before its rows are hashed (all
+// together, 48 BabyBear traces of 2^30.9 cells took 408.5 instead of 406.4 ms).
+constexpr uint64_t kLdeTogetherCells = 1ull << 24;
+
 pico_status enqueue_commit(pico_ctx* ctx, const CommitPlan& plan, cudaStream_t st, cudaStream_t cst,
                            pico_commit* c, std::vector<void*>& scratch, uint32_t* root_host) {
   CommitSetup cs;
@@ -1153,7 +1158,19 @@ pico_status enqueue_commit(pico_ctx* ctx, const CommitPlan& plan, cudaStream_t s
     return PICO_OK;
   };
   uint32_t* layer = c->layers;
+  // Device inputs in the batched form: the LDEs of the shorter groups (whose
+  // rows are hashed together before the tallest group) share launches, and a
+  // small commit's all of them.  With a call per group, each group's power
+  // tables and short passes ran alone.
+  const bool lde_together = !copy_in && !plan.plain && plan.extend;
+  const bool lde_all = lde_together && plan.cells <= kLdeTogetherCells;
+  if (lde_together && (lde_all || G > 1)) {
+    const uint32_t first = lde_all ? 0 : plan.groups[1].first;
+    if ((s = begin_phase(pico_commit::kLde)) || (s = lde_mats(first, (uint32_t)plan.mats.size())) || (s = end_phase()))
+      return s;
+  }
   for (uint32_t gi = G; gi-- > 0 && !s;) {
+    const bool lde_done = lde_all || (lde_together && gi > 0);
     const uint32_t first = plan.groups[gi].first, last = plan.groups[gi].second;
     const uint64_t rows = 1ull << plan.mats[first].log_N;
     uint32_t* digests = gi == 0 ? layer : inj[gi];
@@ -1161,7 +1178,8 @@ pico_status enqueue_commit(pico_ctx* ctx, const CommitPlan& plan, cudaStream_t s
     if (gi == 0 && (s = flush_batch())) break;
     if (!chained[gi]) {
       if (copy_in && (s = cuda_status(cudaStreamWaitEvent(st, arrived[last - 1], 0), "wait for inputs"))) break;
-      if ((s = begin_phase(pico_commit::kLde)) || (s = lde_mats(first, last)) || (s = end_phase())) break;
+      if (!lde_done && ((s = begin_phase(pico_commit::kLde)) || (s = lde_mats(first, last)) || (s = end_phase())))
+        break;
       if (gi > 0 && !plan.plain) {
         if ((s = add_to_batch(first, last, rows, digests))) break;
         continue;
@@ -1180,7 +1198,7 @@ pico_status enqueue_commit(pico_ctx* ctx, const CommitPlan& plan, cudaStream_t s
       if (plan.mats[k].w == 0) continue;
       left--;
       if (copy_in && (s = cuda_status(cudaStreamWaitEvent(st, arrived[k], 0), "wait for inputs"))) break;
-      if ((s = begin_phase(pico_commit::kLde)) || (s = lde_mats(k, k + 1)) || (s = end_phase())) break;
+      if (!lde_done && ((s = begin_phase(pico_commit::kLde)) || (s = lde_mats(k, k + 1)) || (s = end_phase()))) break;
       RowGroup g;
       make_group(k, k + 1, g);
       if ((s = begin_phase(hash_kind))) break;

@@ -578,13 +578,10 @@ __device__ __forceinline__ void forward_from_regs(uint32_t* buf, const uint32_t*
 // ---------------------------------------------------------------------------
 // One-pass form: tile = all n rows of up to LW columns.
 template <class F, int LOG_L>
-__global__ void __launch_bounds__(kThreads, 1) k_lde_small(const __grid_constant__ LdeBatch batch,
-                                                           const __grid_constant__ TwiddleTables tw) {
+__device__ __forceinline__ void lde_small(const LdeMat& M, uint32_t local, const TwiddleTables& tw) {
   constexpr int LOG_LW = (int)tile_log_lw(LOG_L);
   constexpr uint32_t L = 1u << LOG_L;
   extern __shared__ uint32_t smem[];
-  uint32_t local;
-  const LdeMat& M = find_tile(batch, kPassSmall, blockIdx.x, local);
   s_in = GuardRange{M.in, M.in + (((uint64_t)M.w << M.log_n))};
   s_out = GuardRange{M.out, M.out + (((uint64_t)M.w << (M.log_n + lde_log_c(M))))};
   s_smem_words = tile_words_l(LOG_L);
@@ -636,6 +633,36 @@ __global__ void __launch_bounds__(kThreads, 1) k_lde_small(const __grid_constant
           });
     }
   }
+}
+
+template <class F, int LOG_L>
+__global__ void __launch_bounds__(kThreads, 1) k_lde_small(const __grid_constant__ LdeBatch batch,
+                                                           const __grid_constant__ TwiddleTables tw) {
+  uint32_t local;
+  const LdeMat& M = find_tile(batch, kPassSmall, blockIdx.x, local);
+  lde_small<F, LOG_L>(M, local, tw);
+}
+// Matrices of several heights in one launch: a CTA runs the code of its
+// matrix's height.  A launch per height takes 11-18 us for a CTA or a few,
+// one after another (a commit of two tiny traces 231 -> 208 us, of 12 traces of
+// 2^9 .. 2^17 rows 2.24 -> 2.15 ms, with the heights' LDEs enqueued together).
+// The longer passes keep a launch per length: switching there cost a 2^20 x 70
+// LDE 2%.
+template <class F>
+__global__ void __launch_bounds__(kThreads, 1) k_lde_small_mixed(const __grid_constant__ LdeBatch batch,
+                                                                 const __grid_constant__ TwiddleTables tw) {
+  uint32_t local;
+  const LdeMat& M = find_tile(batch, kPassSmall, blockIdx.x, local);
+  switch (M.log_n) {
+#define PICO_LDE_CASE(l)          \
+  case l:                         \
+    lde_small<F, l>(M, local, tw); \
+    break;
+    PICO_LDE_CASE(0) PICO_LDE_CASE(1) PICO_LDE_CASE(2) PICO_LDE_CASE(3) PICO_LDE_CASE(4) PICO_LDE_CASE(5)
+    PICO_LDE_CASE(6) PICO_LDE_CASE(7) PICO_LDE_CASE(8) PICO_LDE_CASE(9) PICO_LDE_CASE(10) PICO_LDE_CASE(11)
+#undef PICO_LDE_CASE
+  }
+  static_assert(kLdeSmallMaxLog == 11, "the cases above");
 }
 
 // Pass A: rows j2 + n2 * j1 of the input -> T1 rows k1 * n2 + j2.
@@ -843,6 +870,9 @@ static cudaError_t set_attrs_from() {
     if ((e = cudaFuncSetAttribute(k_lde_b<F, LOG_L>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap))) return e;
     if ((e = cudaFuncSetAttribute(k_lde_c<F, LOG_L>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap))) return e;
   }
+  if constexpr (LOG_L == 0) {
+    if ((e = cudaFuncSetAttribute(k_lde_small_mixed<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap))) return e;
+  }
   if constexpr (LOG_L < kMaxLogL) e = set_attrs_from<F, LOG_L + 1>();
   return e;
 }
@@ -902,8 +932,33 @@ static cudaError_t launch_lde_t(const LdeMat* mats, uint32_t n_mats, TwiddleTabl
     k_pow_tables<F><<<pgrid, 256, 0, st>>>(all, tw);
     if ((e = cudaGetLastError())) return e;
     if (launches) *launches += 1;
-    // passes in order; within a pass one launch per sub-transform length
-    for (int pass = kPassSmall; pass <= kPassC; pass++) {
+    // the one-pass matrices: one launch, whatever their heights
+    {
+      LdeBatch sub;
+      memset(&sub, 0, sizeof sub);
+      uint32_t tiles = 0;
+      size_t smem = 0;
+      bool mixed = false;
+      for (uint32_t k = 0; k < all.n; k++) {
+        const uint32_t t = lde_tiles(all.m[k], kPassSmall);
+        if (!t) continue;
+        mixed = mixed || (sub.n && sub.m[0].log_n != all.m[k].log_n);
+        sub.m[sub.n++] = all.m[k];
+        tiles += t;
+        smem = std::max(smem, smem_bytes(all.m[k].log_n, kPassSmall));
+      }
+      if (tiles) {
+        if (mixed)
+          k_lde_small_mixed<F><<<tiles, kThreads, smem, st>>>(sub, tw);
+        else
+          launch_pass<F>(sub.m[0].log_n, kPassSmall, tiles, smem, sub, tw, st);
+        if ((e = cudaGetLastError())) return e;
+        if (launches) *launches += 1;
+      }
+    }
+    // three-pass matrices: passes in order, within a pass one launch per
+    // sub-transform length
+    for (int pass = kPassA; pass <= kPassC; pass++) {
       for (uint32_t lL = 0; lL <= (uint32_t)kMaxLogL; lL++) {
         LdeBatch sub;
         memset(&sub, 0, sizeof sub);
