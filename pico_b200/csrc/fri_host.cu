@@ -44,7 +44,7 @@ pico_status enqueue_fri_rounds(int field, cudaStream_t st, const TwiddleTables& 
     while (log_nodes > kSubtreeMaxLog) {
       const uint64_t n = 1ull << log_nodes;
       uint32_t* next = layer + n * 8;
-      if ((s = cuda_status(launch_compress(field, layer, next, n / 2, nullptr, st), "FRI compression"))) return s;
+      if ((s = cuda_status(launch_compress(field, layer, next, n / 2, nullptr, st, true), "FRI compression"))) return s;
       nl++;
       layer = next;
       log_nodes--;
@@ -53,7 +53,7 @@ pico_status enqueue_fri_rounds(int field, cudaStream_t st, const TwiddleTables& 
       const uint32_t levels = subtree_log_in(log_nodes);
       top = levels == log_nodes;
       if ((s = cuda_status(launch_subtree(field, layer, 1u << log_nodes, 1u << levels, SubtreeInj{}, st,
-                                          top ? d_ch : nullptr, d_betas + 4 * r),
+                                          top ? d_ch : nullptr, d_betas + 4 * r, true),
                            "FRI subtree")))
         return s;
       nl++;
@@ -314,14 +314,15 @@ pico_status shard_tree_root(pico_fri_shard* fs, uint32_t root[8]) {
   while (log_nodes > kSubtreeMaxLog) {
     const uint64_t n = 1ull << log_nodes;
     uint32_t* next = layer + n * 8;
-    if ((s = cuda_status(launch_compress(fs->field, layer, next, n / 2, nullptr, fs->st), "FRI compression")))
+    if ((s = cuda_status(launch_compress(fs->field, layer, next, n / 2, nullptr, fs->st, true), "FRI compression")))
       return s;
     layer = next;
     log_nodes--;
   }
   while (log_nodes > 0) {
     const uint32_t levels = subtree_log_in(log_nodes);
-    if ((s = cuda_status(launch_subtree(fs->field, layer, 1u << log_nodes, 1u << levels, SubtreeInj{}, fs->st),
+    if ((s = cuda_status(launch_subtree(fs->field, layer, 1u << log_nodes, 1u << levels, SubtreeInj{}, fs->st, nullptr,
+                                        nullptr, true),
                          "FRI subtree")))
       return s;
     for (uint32_t l = 0; l < levels; l++) layer += (8ull << log_nodes) >> l;

@@ -722,13 +722,12 @@ constexpr uint64_t kTcWholeChunks = 4;
 // Launch a tensor-core kernel over `tiles` tiles: a full wave of CTAs, each
 // looping over its share, or (whole) a CTA per kTcGroups tiles.
 template <class... P, class... A>
-static cudaError_t tc_launch(void (*kernel)(P...), uint64_t tiles, bool whole, cudaStream_t st, A... args) {
+static cudaError_t tc_launch(bool chained, void (*kernel)(P...), uint64_t tiles, bool whole, cudaStream_t st, A... args) {
   uint64_t ctas = tiles;
   if (ctas > kTcResident) ctas = whole ? std::max<uint64_t>((tiles + kTcGroups - 1) / kTcGroups, kTcResident) : kTcResident;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmemBytes);
   if (e) return e;
-  kernel<<<(unsigned)ctas, kTcThreads * kTcGroups, kTcSmemBytes, st>>>(args...);
-  return cudaGetLastError();
+  return launch_chained(chained, kernel, (unsigned)ctas, kTcThreads * kTcGroups, kTcSmemBytes, st, args...);
 }
 
 // ---------------------------------------------------------------------------
@@ -764,7 +763,7 @@ cudaError_t launch_permute(int field, uint32_t* states, uint64_t n, cudaStream_t
     return cudaGetLastError();
   }
   if (n >= kTcMinStates) {
-    return tc_launch(field == 0 ? k_permute_tc<KoalaBear> : k_permute_tc<BabyBear>, tc_tiles(n), false, st, states,
+    return tc_launch(false, field == 0 ? k_permute_tc<KoalaBear> : k_permute_tc<BabyBear>, tc_tiles(n), false, st, states,
                      n);
   }
   if (field == 0)
@@ -828,15 +827,12 @@ cudaError_t launch_hash_groups(int field, const GroupBatch& b, cudaStream_t st, 
     chunks += t * ((b.width[g] + 7) / 8);
   }
   if (use_tensor_rows(rows, chunks / tiles)) {
-    return tc_launch(field == 0 ? k_hash_groups_tc<KoalaBear> : k_hash_groups_tc<BabyBear>, tiles,
+    return tc_launch(false, field == 0 ? k_hash_groups_tc<KoalaBear> : k_hash_groups_tc<BabyBear>, tiles,
                      chunks >= kTcWholeChunks * tiles, st, b, tiles);
   }
   if (rows <= kLaneMaxStates) {
-    if (field == 0)
-      k_hash_groups_lane<KoalaBear><<<blocks_for(16 * rows, kLaneThreads), kLaneThreads, 0, st>>>(b);
-    else
-      k_hash_groups_lane<BabyBear><<<blocks_for(16 * rows, kLaneThreads), kLaneThreads, 0, st>>>(b);
-    return cudaGetLastError();
+    return launch_chained(false, field == 0 ? k_hash_groups_lane<KoalaBear> : k_hash_groups_lane<BabyBear>,
+                          blocks_for(16 * rows, kLaneThreads), kLaneThreads, 0, st, b);
   }
   if (block < 32 || block > 256) block = 256;
   if (field == 0)
@@ -851,17 +847,13 @@ cudaError_t launch_absorb_rows(int field, const RowGroup& g, uint64_t rows, uint
   if (rows == 0) return cudaSuccess;
   const uint64_t absorbed = pos0 + g.total_width;
   if (use_tensor_rows(rows, absorbed / 8)) {
-    return tc_launch(field == 0 ? k_absorb_rows_tc<KoalaBear> : k_absorb_rows_tc<BabyBear>, tc_tiles(rows), absorbed >= 8 * kTcWholeChunks, st,
+    return tc_launch(false, field == 0 ? k_absorb_rows_tc<KoalaBear> : k_absorb_rows_tc<BabyBear>, tc_tiles(rows),
+                     absorbed >= 8 * kTcWholeChunks, st,
                      g, rows, pos0, state_in, state_out, digest_out);
   }
   if (rows <= kLaneMaxStates) {
-    if (field == 0)
-      k_absorb_rows_lane<KoalaBear><<<blocks_for(16 * rows, kLaneThreads), kLaneThreads, 0, st>>>(
-          g, rows, pos0, state_in, state_out, digest_out);
-    else
-      k_absorb_rows_lane<BabyBear><<<blocks_for(16 * rows, kLaneThreads), kLaneThreads, 0, st>>>(
-          g, rows, pos0, state_in, state_out, digest_out);
-    return cudaGetLastError();
+    return launch_chained(false, field == 0 ? k_absorb_rows_lane<KoalaBear> : k_absorb_rows_lane<BabyBear>,
+                          blocks_for(16 * rows, kLaneThreads), kLaneThreads, 0, st, g, rows, pos0, state_in, state_out, digest_out);
   }
   if (block < 32 || block > 256) block = 256;
   if (field == 0)
@@ -904,14 +896,11 @@ __global__ void __launch_bounds__(256) k_compress_quad(const uint32_t* prev, uin
 }
 
 cudaError_t launch_compress(int field, const uint32_t* prev, uint32_t* next, uint64_t n_next,
-                            const uint32_t* inj_digests, cudaStream_t st) {
+                            const uint32_t* inj_digests, cudaStream_t st, bool chained) {
   if (n_next == 0) return cudaSuccess;
   if (n_next <= kLaneMaxStates) {
-    if (field == 0)
-      k_compress_lane<KoalaBear><<<blocks_for(16 * n_next, kLaneThreads), kLaneThreads, 0, st>>>(prev, next, n_next, inj_digests);
-    else
-      k_compress_lane<BabyBear><<<blocks_for(16 * n_next, kLaneThreads), kLaneThreads, 0, st>>>(prev, next, n_next, inj_digests);
-    return cudaGetLastError();
+    return launch_chained(chained, field == 0 ? k_compress_lane<KoalaBear> : k_compress_lane<BabyBear>,
+                          blocks_for(16 * n_next, kLaneThreads), kLaneThreads, 0, st, prev, next, n_next, inj_digests);
   }
   if (n_next <= kQuadMaxNodes) {
     if (field == 0)
@@ -921,7 +910,7 @@ cudaError_t launch_compress(int field, const uint32_t* prev, uint32_t* next, uin
     return cudaGetLastError();
   }
   if (n_next >= kTcMinStates) {
-    return tc_launch(field == 0 ? k_compress_tc<KoalaBear> : k_compress_tc<BabyBear>, tc_tiles(n_next), false, st,
+    return tc_launch(chained, field == 0 ? k_compress_tc<KoalaBear> : k_compress_tc<BabyBear>, tc_tiles(n_next), false, st,
                      prev, next, n_next, inj_digests);
   }
   if (field == 0)
@@ -1108,13 +1097,9 @@ __global__ void __launch_bounds__(kTcThreads * kTcGroups, kTcCtas)
 static cudaError_t launch_fri_fold_hash_lane(int field, const uint32_t* cw, uint32_t log_len, uint64_t row0, uint64_t n,
                                              const uint32_t* beta, TwiddleTables tw, uint32_t* out,
                                              const uint32_t* inject, uint32_t* leaves, cudaStream_t st) {
-  if (field == 0)
-    k_fri_fold_hash_lane<KoalaBear><<<blocks_for(16 * n, kLaneThreads), kLaneThreads, 0, st>>>(cw, log_len, row0, n, beta,
-                                                                                              tw, out, inject, leaves);
-  else
-    k_fri_fold_hash_lane<BabyBear><<<blocks_for(16 * n, kLaneThreads), kLaneThreads, 0, st>>>(cw, log_len, row0, n, beta,
-                                                                                             tw, out, inject, leaves);
-  return cudaGetLastError();
+  return launch_chained(true, field == 0 ? k_fri_fold_hash_lane<KoalaBear> : k_fri_fold_hash_lane<BabyBear>,
+                        blocks_for(16 * n, kLaneThreads), kLaneThreads, 0, st, cw, log_len, row0, n, beta, tw, out, inject,
+                        leaves);
 }
 
 cudaError_t launch_fri_fold_hash_rows(int field, const uint32_t* cw, uint32_t log_len, uint64_t row0,
@@ -1123,7 +1108,7 @@ cudaError_t launch_fri_fold_hash_rows(int field, const uint32_t* cw, uint32_t lo
   if (n_leaves == 0) return cudaSuccess;
   if (log_len < 2 || 2 * (row0 + 2 * n_leaves) > (1ull << log_len)) return cudaErrorInvalidValue;
   if (n_leaves >= kTcMinStates)
-    return tc_launch(field == 0 ? k_fri_fold_hash_tc<KoalaBear> : k_fri_fold_hash_tc<BabyBear>, tc_tiles(n_leaves), false,
+    return tc_launch(true, field == 0 ? k_fri_fold_hash_tc<KoalaBear> : k_fri_fold_hash_tc<BabyBear>, tc_tiles(n_leaves), false,
                      st, cw, log_len, row0, n_leaves, beta, tw, out, (const uint32_t*)nullptr, leaves);
   if (n_leaves <= kLaneMaxStates)
     return launch_fri_fold_hash_lane(field, cw, log_len, row0, n_leaves, beta, tw, out, nullptr, leaves, st);
@@ -1142,7 +1127,7 @@ cudaError_t launch_fri_fold_hash(int field, const uint32_t* cw, uint32_t log_len
   if (log_len < 2) return cudaErrorInvalidValue;
   const uint64_t n = 1ull << (log_len - 2);
   if (n >= kTcMinStates)
-    return tc_launch(field == 0 ? k_fri_fold_hash_tc<KoalaBear> : k_fri_fold_hash_tc<BabyBear>, tc_tiles(n), false, st, cw,
+    return tc_launch(true, field == 0 ? k_fri_fold_hash_tc<KoalaBear> : k_fri_fold_hash_tc<BabyBear>, tc_tiles(n), false, st, cw,
                      log_len, (uint64_t)0, n, beta, tw, out, inject, leaves);
   if (n <= kLaneMaxStates)
     return launch_fri_fold_hash_lane(field, cw, log_len, 0, n, beta, tw, out, inject, leaves, st);
@@ -1164,22 +1149,16 @@ cudaError_t launch_fri_fold_tw(int field, const uint32_t* cw, uint32_t log_len, 
 }
 
 cudaError_t launch_subtree(int field, uint32_t* level, uint32_t n_in, uint32_t n, const SubtreeInj& inj,
-                           cudaStream_t st, DevChallenger* ch, uint32_t* beta_out) {
+                           cudaStream_t st, DevChallenger* ch, uint32_t* beta_out, bool chained) {
   if (n == 0 || n > kSubtreeMaxIn || (n & (n - 1)) || n_in % n || (ch && n != n_in)) return cudaErrorInvalidValue;
-  if (field == 0)
-    k_subtree_lane<KoalaBear><<<n_in / n, kSubtreeThreads, 0, st>>>(level, n_in, n, inj, ch, beta_out);
-  else
-    k_subtree_lane<BabyBear><<<n_in / n, kSubtreeThreads, 0, st>>>(level, n_in, n, inj, ch, beta_out);
-  return cudaGetLastError();
+  return launch_chained(chained, field == 0 ? k_subtree_lane<KoalaBear> : k_subtree_lane<BabyBear>, n_in / n, kSubtreeThreads, 0, st,
+                        level, n_in, n, inj, ch, beta_out);
 }
 
 cudaError_t launch_challenger_observe(int field, DevChallenger* ch, const uint32_t* vals, uint32_t n,
                                       cudaStream_t st) {
-  if (field == 0)
-    k_challenger_observe<KoalaBear><<<1, 32, 0, st>>>(ch, vals, n);
-  else
-    k_challenger_observe<BabyBear><<<1, 32, 0, st>>>(ch, vals, n);
-  return cudaGetLastError();
+  return launch_chained(true, field == 0 ? k_challenger_observe<KoalaBear> : k_challenger_observe<BabyBear>, 1, 32, 0, st, ch, vals,
+                        n);
 }
 
 // Proof-of-work search (the challenger's grind; checked by check_witness,

@@ -24,6 +24,7 @@
 //   16 requests of ~20 small traces 4.78 -> 4.35 ms.
 #pragma once
 #include "field.cuh"
+#include "internal.h"
 #include "p2_layers.cuh"
 #include "p2_tc_tables.h"
 
@@ -31,11 +32,14 @@ namespace pico {
 
 __device__ uint32_t g_p2_lane[2][kLaneWords];
 
-// Copy a field's tables to shared memory (the caller synchronises).
+// Copy a field's tables to shared memory (the caller synchronises) and wait
+// for the kernel before this one.
 template <class F>
 __device__ __forceinline__ void lane_load_tables(uint32_t* tab) {
   const uint4* src = reinterpret_cast<const uint4*>(g_p2_lane[F::ID]);
+  grid_release();
   for (uint32_t i = threadIdx.x; i < kLaneWords / 4; i += blockDim.x) reinterpret_cast<uint4*>(tab)[i] = __ldg(src + i);
+  grid_wait();
 }
 
 // 64-bit sums of products of canonical values: four fit (4 p^2 < 2^64); a fold

@@ -387,6 +387,7 @@ struct P2Tc {
   // Set-up and tear-down, by the whole CTA: tables into shared memory, TMEM
   // columns, a barrier per group, the constant word.
   __device__ __forceinline__ void open(uint8_t* tables, uint64_t* mbar, uint32_t* tmem_slot) {
+    grid_release();
     const uint4* src = g_p2_tc[F::ID];
     for (uint32_t i = threadIdx.x; i < kTcTableBytes / 16; i += kTcThreads * kTcGroups)
       reinterpret_cast<uint4*>(tables)[i] = __ldg(src + i);
@@ -417,6 +418,7 @@ struct P2Tc {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     tmem = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(tmem_slot), 0) + kTcCols * group;
     lane = tmem + ((warp % 4) << 21);
+    grid_wait();
   }
   __device__ __forceinline__ void close() {
     __syncwarp();
