@@ -144,11 +144,11 @@ def peaks():
     return 6650.0, "fallback"
 
 
-# Algorithmic Poseidon2 work: modular multiplications per permutation (S-box
-# products plus one internal-diagonal product per lane per partial round;
-# additions excluded): KoalaBear 8*16*2 + 20*2 + 20*16, BabyBear
-# 8*16*4 + 13*4 + 13*16.  One Montgomery product ~ 4 IMAD-pipe instructions.
-PERM_MODMULS = {0: 8 * 16 * 2 + 20 * 2 + 20 * 16, 1: 8 * 16 * 4 + 13 * 4 + 13 * 16}
+# Algorithmic Poseidon2 work on the integer multiplier: the S-box products of
+# a permutation, KoalaBear (8*16 + 20)*2, BabyBear (8*16 + 13)*4 (the linear
+# layers, the internal diagonal included, are tensor-core products).  One
+# Montgomery product ~ 4 IMAD-pipe instructions.
+PERM_MODMULS = {0: (8 * 16 + 20) * 2, 1: (8 * 16 + 13) * 4}
 IMAD_PER_MODMUL = 4
 IMAD_PER_SM_CLK = 64
 # DRAM bytes per algorithmic byte of one leaf-hashing launch (dram__bytes_read
@@ -456,7 +456,7 @@ def run_gpu(args, rank, world, local):
         "gpu_launches": int(sum(s["launches"] for s in stats)),
         "clocks": clocks,
         "roofline": {
-            "kernel": "k_hash_rows (Poseidon2 leaf hashing, one launch per commit)",
+            "kernel": "k_hash_groups_tc (Poseidon2 leaf hashing, one launch per commit)",
             "bound": "imad",
             "achieved": imad_ach,
             "peak": imad_peak,
@@ -465,7 +465,7 @@ def run_gpu(args, rank, world, local):
             "traffic": leaf_bytes * HASH_TRAFFIC_RATIO,
             "algorithmic_bytes": leaf_bytes,
             "launch_ms": leaves_s * 1e3,
-            "note": f"integer-multiply bound: achieved = {IMAD_PER_MODMUL} IMAD x {PERM_MODMULS[field]} modmuls "
+            "note": f"integer-multiply bound: achieved = {IMAD_PER_MODMUL} IMAD x {PERM_MODMULS[field]} S-box products "
                     f"x leaf permutations / launch time; peak = {sm_count} SMs x {IMAD_PER_SM_CLK} IMAD/clk x "
                     f"median SM clock; traffic = algorithmic bytes x the DRAM/algorithmic ratio ncu measured",
         },
@@ -858,10 +858,10 @@ def run_fri(args):
         "gpu_launches": args.steps * fri_launches(log_trace + b, rounds, 0),
         "e2e": {"value": n_el / e2e_s, "unit": "elements/s", "ms_per_step": e2e_s * 1e3,
                 "h2d_bytes_per_step": n_el * 16, "d2h_bytes_per_step": rounds * 48 + 16},
-        "roofline": {"kernel": "the phase's Poseidon2 kernels (k_fri_fold_hash, k_compress, k_subtree_quad, "
-                               "k_tree_top)", "bound": "imad", "achieved": imad_ach, "peak": imad_peak,
+        "roofline": {"kernel": "the phase's Poseidon2 kernels (k_fri_fold_hash*, k_compress*, k_subtree_lane)",
+                     "bound": "imad", "achieved": imad_ach, "peak": imad_peak,
                      "unit": "Tops/s", "frac": imad_ach / imad_peak, "traffic": None, "permutations": perms,
-                     "note": "survey model: 4 IMAD x modmuls per permutation; the phase is bound by chains of "
+                     "note": "4 IMAD x S-box products per permutation; the phase is bound by chains of "
                              "dependent permutations (each round's leaves need the previous round's beta)"},
         "cpu_baseline": {"value": (1 << (small + b)) / cpu_s, "unit": "elements/s", "cores": orc.num_threads(),
                          "kind": "port", "cpu_model": cpu_model(),
