@@ -63,14 +63,14 @@ cudaError_t upload_p2_constants(int field, const uint32_t ext[8][16], const uint
 // 2^17 46.2 / 39.1, 2^20 226 / 160.  Below, the latency of one permutation
 // sets the time, and the table load and product stages make it longer.
 constexpr uint64_t kTcMinStates = 1u << 16;
-// Rows of several permutations each: from here on (a row's chain, 2^14 rows of
-// 64 columns: 47 us one thread per row, 38 on the tensor cores).
+// Rows of several permutations each: from here on.  16 requests of ~20 small
+// traces took 4.78 ms with 2^16, 4.94 with 2^15, 4.49 with 2^14 and 4.39 with
+// 2^13 (runs of one build differ by 0.15 ms, so the last two are equal).
 constexpr uint64_t kTcMinRows = 1u << 13;
 // four_lanes: four threads per state (the latency form).
 cudaError_t launch_permute(int field, uint32_t* states, uint64_t n, cudaStream_t st, bool four_lanes = false);
-// At most this many states: 16 lanes per state (p2_lane.cuh), bound by latency
-// up to ~2^12 states and by issue above (1.2 G/s against 5 G/s one thread per
-// state); with 2^14 a FRI phase of 2^23 elements took 4.20 instead of 4.11 ms.
+// At most this many states: 16 lanes per state (p2_lane.cuh).  A FRI phase of
+// 2^23 elements took 4.20 ms with 2^14, 4.11 with this and 4.12 with 2^12.
 constexpr uint64_t kLaneMaxStates = 8192;
 // Levels of at most this many nodes are compressed four threads per node.
 constexpr uint64_t kQuadMaxNodes = 16384;
@@ -112,9 +112,8 @@ cudaError_t launch_subtree(int field, uint32_t* level, uint32_t n_in, uint32_t n
 // The narrow levels of a tree, from 2^log_n <= 2^kSubtreeMaxLog nodes to the
 // root: nodes per CTA (log) of the next launch.  Up to 2^7 nodes go in one
 // launch; above, one over many CTAs leaves 2^6 (from 2^14, 2^7) for another.
-// A level costs its 1.9 us of latency while a CTA has at most 32 nodes to make
-// (two per warp), twice that at 64; a further launch costs about as much as
-// one level.
+// A level costs one permutation's latency (4,000 cycles, 2 us) while a CTA has
+// at most 32 nodes to make (two per warp), twice that at 64.
 constexpr uint32_t kSubtreeMaxLog = 14;
 inline uint32_t subtree_log_in(uint32_t log_n) { return log_n <= 7 ? log_n : log_n <= 13 ? log_n - 6 : 7; }
 // next[i] = compress(prev[2i], prev[2i+1]); if inj_digests != null:

@@ -16,12 +16,11 @@
 // Latency of one permutation in cycles, one thread / four lanes / this form:
 // KoalaBear 11,270 / 8,400 / about 4,200, BabyBear 16,020 / 7,950 / 3,960.  In a full
 // round the two shuffle steps and their six dependent additions take 115
-// cycles and the S-box 50 (90); a partial round 65 (105); the sums before
-// them 450.  Unrolled partial rounds (8 KB of code) measured 5% faster on a
-// FRI phase than loops of three, whose table loads are not hidden.
+// cycles and the S-box 50 (90).  Unrolled partial rounds: a FRI phase of 4.04
+// ms, against 4.25 with loops of three.
 //   commit of 2 tiny BabyBear traces 314 -> 231 us, 2^16 x 64 commit 504 -> 481 us,
 //   FRI phase of 2^23 elements 4.70 -> 4.04 ms, opening of 2^26 cells 3.70 -> 3.17 ms,
-//   16 requests of ~20 small traces 4.78 -> 4.35 ms.
+//   16 requests of ~20 small traces 4.78 -> 4.3..4.6 ms.
 #pragma once
 #include "field.cuh"
 #include "internal.h"

@@ -23,7 +23,8 @@
 //     z and earlier blocks, and the y of the same block are added by
 //     multiply-accumulates in registers.
 //
-// Bound: the multiplier pipe (fmaheavy 68% busy; issue 50%) and the latency of
+// Bound: the multiplier pipe (hashing 2^17 rows
+// of 64 columns: fmaheavy 57% busy, issue 47%) and the latency of
 // the 24 product stages of a permutation (~280 cycles each alone: barrier,
 // products, commit, read-back), which the eight groups of an SM overlap.
 // Layout: the accumulators hold half a layer (32 columns), so that z (32
