@@ -978,7 +978,7 @@ def run_quotient(args):
         "parity": {"matches_oracle": match, "points": points},
         "clocks": clocks,
         "gpu_launches": args.steps,
-        "roofline": {"kernel": "k_quotient", "bound": "hbm", "achieved": q_ach, "peak": hbm_peak, "unit": "GB/s",
+        "roofline": {"kernel": "k_quotient_staged", "bound": "hbm", "achieved": q_ach, "peak": hbm_peak, "unit": "GB/s",
                      "frac": q_ach / hbm_peak, "traffic": None, "algorithmic_bytes": q_bytes,
                      "peak_source": f"{hbm_kind} (MEASURED_PEAKS.json hbm_gbs)" if hbm_kind == "measured" else "fallback",
                      "note": "the kernel interprets the constraint program per point, so its instruction stream, not "
