@@ -30,6 +30,11 @@ struct RowGroup {
 // each loads its constant tables first and waits for the previous kernel to
 // be complete (grid_wait) before it touches any other memory; grid_release
 // lets the next one start.  Both do nothing in a kernel launched normally.
+// A kernel that may be chained reads what other kernels write with ordinary
+// loads, after grid_wait: __ldg (ld.global.nc) is defined only for memory that
+// nothing writes in the reading kernel's whole life, which here begins before
+// its input is complete, and may be moved above the wait.  __ldg is for the
+// constant tables.
 // FRI phase of 2^23 elements 4.09 -> 3.86 ms, opening of 2^26 cells 3.16 -> 3.06.
 // Commits launch normally: there it gave 0.5%, and among served requests the
 // waiting kernels hold the SMs other streams could use (16 small requests 4.16

@@ -268,9 +268,9 @@ __global__ void __launch_bounds__(kLaneThreads) k_compress_lane(const uint32_t* 
   const uint64_t i = t >> 4;
   const uint32_t q = (uint32_t)(t & 15);
   const bool live = i < n;
-  uint32_t v = live ? __ldg(prev + 16 * i + q) : 0u;
+  uint32_t v = live ? prev[16 * i + q] : 0u;
   uint32_t d = 0;
-  if (inj && live && q >= 8) d = __ldg(inj + 8 * i + q - 8);
+  if (inj && live && q >= 8) d = inj[8 * i + q - 8];
   __syncthreads();
   v = lane_permute<F>(v, q, tab);
   if (inj) {
@@ -422,7 +422,7 @@ __device__ __forceinline__ uint32_t* lane_subtree(uint32_t* cur, uint32_t* spare
       const bool live = node < m;
       uint32_t v = live ? cur[16 * node + q] : 0u;
       uint32_t w = 0;
-      if (d && live && q >= 8) w = __ldg(d + (c * m + node) * 8 + q - 8);
+      if (d && live && q >= 8) w = d[(c * m + node) * 8 + q - 8];
       v = lane_permute<F>(v, q, tab);
       if (d) {
         if (q >= 8) v = w;
@@ -688,7 +688,7 @@ __global__ void __launch_bounds__(kTcThreads * kTcGroups, kTcCtas)
     const uint4* p = reinterpret_cast<const uint4*>(prev + 16 * ii);
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-      const uint4 v = __ldg(p + k);
+      const uint4 v = p[k];
       s[4 * k] = v.x;
       s[4 * k + 1] = v.y;
       s[4 * k + 2] = v.z;
@@ -700,7 +700,7 @@ __global__ void __launch_bounds__(kTcThreads * kTcGroups, kTcCtas)
       tc.digest(s);
       if (!inj || pass) break;
       const uint4* q = reinterpret_cast<const uint4*>(inj + 8 * ii);
-      const uint4 a = __ldg(q), c = __ldg(q + 1);
+      const uint4 a = q[0], c = q[1];
       s[8] = a.x;
       s[9] = a.y;
       s[10] = a.z;
@@ -930,7 +930,8 @@ cudaError_t launch_compress(int field, const uint32_t* prev, uint32_t* next, uin
 //   (lo + hi)/2 + (beta/2) * g_inv^rev(r) * (lo - hi),
 // g = two_adic_generator(log len), rev over log(len/2) bits.  The pair is read
 // at rows 2r, 2r+1 of cw; rg is its row in the whole codeword (r itself,
-// except for one shard of a codeword split by rows).
+// except for one shard of a codeword split by rows).  Ordinary loads here and
+// in half_beta: chained kernels call both (launch_chained).
 template <class F>
 __device__ __forceinline__ Ext4 fri_fold_row(const uint32_t* cw, uint32_t log_len, uint64_t r, const Ext4& hb,
                                              const TwiddleTables& tw, uint64_t rg) {
@@ -941,8 +942,8 @@ __device__ __forceinline__ Ext4 fri_fold_row(const uint32_t* cw, uint32_t log_le
   uint32_t e = (uint32_t)bitrev64(rg, (int)log_len - 1) << (F::TWO_ADICITY - log_len);
   e = (0u - e) & mask;
   uint32_t t = B::mul(__ldg(tw.hi + (e >> 14)), __ldg(tw.lo + (e & 0x3fffu)));
-  const uint4 lo4 = __ldg(reinterpret_cast<const uint4*>(cw) + 2 * r);
-  const uint4 hi4 = __ldg(reinterpret_cast<const uint4*>(cw) + 2 * r + 1);
+  const uint4 lo4 = reinterpret_cast<const uint4*>(cw)[2 * r];
+  const uint4 hi4 = reinterpret_cast<const uint4*>(cw)[2 * r + 1];
   Ext4 lo{{lo4.x, lo4.y, lo4.z, lo4.w}}, hi{{hi4.x, hi4.y, hi4.z, hi4.w}};
   Ext4 sum = E::add(lo, hi), dif = E::sub(lo, hi);
   Ext4 res;
@@ -956,7 +957,7 @@ template <class F>
 __device__ __forceinline__ Ext4 half_beta(const uint32_t* beta) {
   Ext4 hb;
 #pragma unroll
-  for (int i = 0; i < 4; i++) hb.c[i] = Fp<F>::half(__ldg(beta + i));
+  for (int i = 0; i < 4; i++) hb.c[i] = Fp<F>::half(beta[i]);
   return hb;
 }
 
@@ -968,7 +969,7 @@ __global__ void k_fri_fold(const uint32_t* cw, uint32_t log_len, const uint32_t*
   if (r >= h) return;
   Ext4 res = fri_fold_row<F>(cw, log_len, r, half_beta<F>(beta), tw, r);
   if (inject) {
-    const uint4 v = __ldg(reinterpret_cast<const uint4*>(inject) + r);
+    const uint4 v = reinterpret_cast<const uint4*>(inject)[r];
     res = Ef<F>::add(res, Ext4{{v.x, v.y, v.z, v.w}});
   }
   reinterpret_cast<uint4*>(out)[r] = make_uint4(res.c[0], res.c[1], res.c[2], res.c[3]);
@@ -991,7 +992,7 @@ __global__ void __launch_bounds__(256) k_fri_fold_hash(const uint32_t* cw, uint3
     const uint64_t r = 2 * k + u;
     Ext4 res = fri_fold_row<F>(cw, log_len, r, hb, tw, r);
     if (inject) {
-      const uint4 v = __ldg(reinterpret_cast<const uint4*>(inject) + r);
+      const uint4 v = reinterpret_cast<const uint4*>(inject)[r];
       res = Ef<F>::add(res, Ext4{{v.x, v.y, v.z, v.w}});
     }
     reinterpret_cast<uint4*>(out)[r] = make_uint4(res.c[0], res.c[1], res.c[2], res.c[3]);
@@ -1052,7 +1053,7 @@ __global__ void __launch_bounds__(kLaneThreads)
     const uint64_t r = 2 * k + (q >> 2);
     const Ext4 res = fri_fold_row<F>(cw, log_len, r, half_beta<F>(beta), tw, row0 + r);
     v = (q & 2) ? ((q & 1) ? res.c[3] : res.c[2]) : ((q & 1) ? res.c[1] : res.c[0]);
-    if (inject) v = Fp<F>::add(v, __ldg(inject + 4 * r + (q & 3)));
+    if (inject) v = Fp<F>::add(v, inject[4 * r + (q & 3)]);
     out[4 * r + (q & 3)] = v;
   }
   __syncthreads();
@@ -1078,7 +1079,7 @@ __global__ void __launch_bounds__(kTcThreads * kTcGroups, kTcCtas)
         const uint64_t r = 2 * k + u;
         Ext4 res = fri_fold_row<F>(cw, log_len, r, hb, tw, row0 + r);
         if (inject) {
-          const uint4 v = __ldg(reinterpret_cast<const uint4*>(inject) + r);
+          const uint4 v = reinterpret_cast<const uint4*>(inject)[r];
           res = Ef<F>::add(res, Ext4{{v.x, v.y, v.z, v.w}});
         }
         reinterpret_cast<uint4*>(out)[r] = make_uint4(res.c[0], res.c[1], res.c[2], res.c[3]);
