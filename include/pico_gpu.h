@@ -484,13 +484,19 @@ pico_status pico_gpu_autotune(pico_ctx *ctx, pico_field field, uint32_t log_n_mi
 pico_status pico_gpu_lde_split(pico_ctx *ctx, pico_field field, uint32_t log_n, uint32_t set_log_n1,
                                uint32_t *log_n1_out);
 
-/* ---- test hook (no counterpart in the reference) ----------------------------
+/* ---- test hooks (no counterpart in the reference) ----------------------------
  * Failure injection on the host: after `after` more device allocations made by
  * this library (any context, any thread), the next one fails as if the device
  * were out of memory (PICO_ERR_OUT_OF_MEMORY), then injection switches off;
  * after < 0 switches it off.  Tests use it to check that a failed commit
  * returns its budget and buffers and leaves the context usable. */
 pico_status pico_gpu_test_fail_allocations(int64_t after);
+/* From now on every wait of the tensor-core Poseidon2 kernels for a product on
+ * the context's device runs out after `tries` tries (tries >= 0), as if the
+ * product never arrived; tries < 0 switches it off.  Nothing else may run on
+ * the device during this call.  Tests use it to check that the calls report a
+ * wait that ran out and leave the context usable. */
+pico_status pico_gpu_test_expire_tensor_waits(pico_ctx *ctx, int64_t tries);
 
 #ifdef __cplusplus
 }

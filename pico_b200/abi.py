@@ -199,6 +199,7 @@ SIGNATURES = {
     "pico_gpu_open_values": (C.c_int, [_vp, C.POINTER(OpenBatch), _u32, _u32, _vp]),
     "pico_gpu_reduced_opening": (C.c_int, [_vp, C.POINTER(OpenBatch), _u32, _u32, _vp, _vp, _u32, _vp]),
     "pico_gpu_test_fail_allocations": (C.c_int, [C.c_int64]),
+    "pico_gpu_test_expire_tensor_waits": (C.c_int, [C.c_void_p, C.c_int64]),
     "pico_gpu_quotient_values": (
         C.c_int,
         [_vp, TraceRef, TraceRef, TraceRef, _u32, _u32, _vp, _u32, _vp, _u32, _vp, _u32, _vp, _vp, _vp, _vp, _u32],

@@ -343,6 +343,15 @@ extern "C" pico_status pico_gpu_test_fail_allocations(int64_t after) {
   return PICO_OK;
 }
 
+extern "C" pico_status pico_gpu_test_expire_tensor_waits(pico_ctx* ctx, int64_t tries) {
+  if (!ctx) {
+    set_error("test_expire_tensor_waits: null context");
+    return PICO_ERR_INVALID_ARG;
+  }
+  cudaSetDevice(ctx->device);
+  return cuda_status(expire_tensor_waits(tries), "test_expire_tensor_waits");
+}
+
 static void free_async(void* p, cudaStream_t st) {
   if (p) cudaFreeAsync(p, st);
 }

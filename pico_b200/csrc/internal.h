@@ -62,6 +62,8 @@ static cudaError_t launch_chained(bool chained, void (*kernel)(P...), unsigned g
 // --- Poseidon2 / Merkle kernels (p2_kernels.cu) -------------------------
 cudaError_t upload_p2_constants(int field, const uint32_t ext[8][16], const uint32_t* inte, int rounds_p,
                                 const uint32_t diag[16]);
+// Tests: let the tensor-core form's waits run out (pico_gpu_test_expire_tensor_waits).
+cudaError_t expire_tensor_waits(int64_t tries);
 // Launches of at least this many states use the tensor-core form (p2_tc.cuh).
 // One permutation of n states, one thread per state against the tensor cores
 // (KoalaBear, host call included): 2^15 23.8 / 29.1 us, 2^16 31.2 / 29.3,

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstddef>
 #include <cstring>
 #include <vector>
 
@@ -32,6 +33,18 @@ cudaError_t upload_p2_constants(int field, const uint32_t ext[8][16], const uint
   if ((e = cudaMemcpyToSymbol(g_p2_lane, lane.data(), kLaneWords * 4, (size_t)kLaneWords * 4 * (field ? 1 : 0)))) return e;
   if ((e = cudaMemcpyToSymbol(g_p2_tc, tables.data(), kTcTableBytes, (size_t)kTcTableBytes * (field ? 1 : 0)))) return e;
   return cudaMemcpyToSymbol(c_p2_tc, &tc, sizeof tc, sizeof tc * (field ? 1 : 0));
+}
+
+// From now on (tries >= 0) a wait for tensor-core products gives up after that
+// many tries and none ever succeeds: the barriers need an arrival that nothing
+// makes.  tries < 0: as built.
+cudaError_t expire_tensor_waits(int64_t tries) {
+  const uint32_t w[2] = {tries < 0 ? kTcWaitTries : (uint32_t)std::min<int64_t>(tries, kTcWaitTries), tries < 0 ? 1u : 2u};
+  static_assert(offsetof(P2TcConstants, arrivals) == offsetof(P2TcConstants, wait_tries) + 4, "copied together");
+  cudaError_t e = cudaSuccess;
+  for (size_t f = 0; f < 2 && !e; f++)
+    e = cudaMemcpyToSymbol(c_p2_tc, w, sizeof w, f * sizeof(P2TcConstants) + offsetof(P2TcConstants, wait_tries));
+  return e ? e : cudaDeviceSynchronize();
 }
 
 // ---------------------------------------------------------------------------

@@ -105,7 +105,7 @@ struct P2Tc {
   uint32_t phase;
   uint32_t warp;   // warp-uniform values, so that the products' operands need no per-thread registers
   uint32_t turn;   // which of the group's warps issues next
-  bool dead;       // a wait ran out: no more products or waits, results are void and reported
+  uint32_t dead;   // not 0: a wait ran out (for phase dead - 1): no more products or waits, results are void and reported
 
   __device__ __forceinline__ uint64_t desc(uint32_t offset, uint32_t lbo) const {
     return (uint64_t)((sm >> 4) + (offset >> 4) + ((lbo >> 4) << 16)) | ((uint64_t)((128u >> 4) | (1u << 14)) << 32);
@@ -158,19 +158,25 @@ struct P2Tc {
     wait();
   }
   __device__ __forceinline__ void wait() {
-    if (!dead) {
-      uint32_t ok = 0;
-#pragma unroll 1
-      for (uint32_t i = 0; i < (1u << 20) && !ok; i++)
-        asm volatile("{.reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p;}"
-                     : "=r"(ok)
-                     : "r"(bar), "r"(phase)
-                     : "memory");
-      dead = __any_sync(0xffffffffu, !ok);
-    }
+    if (!dead && __any_sync(0xffffffffu, !arrived(phase))) dead = 1 + phase;
     __syncwarp();
     phase ^= 1;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  }
+  // Whether the products of a phase have arrived, after a bounded wait.
+  __device__ __forceinline__ bool arrived(uint32_t parity) const {
+    auto tried = [&] {
+      uint32_t ok;
+      asm volatile("{.reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p;}"
+                   : "=r"(ok)
+                   : "r"(bar), "r"(parity)
+                   : "memory");
+      return ok != 0;
+    };
+    bool ok = tried();
+#pragma unroll 1
+    for (uint32_t i = 1; !ok && i < c_p2_tc[F::ID].wait_tries; i++) ok = tried();
+    return ok;
   }
 
   // ---- arithmetic: signed Montgomery values ---------------------------------
@@ -401,7 +407,7 @@ struct P2Tc {
       reinterpret_cast<uint4*>(tables + kTcOne)[i] = make_uint4(0u, 0u, 0u, i >= kTcStepBytes / 32 ? 1u : 0u);
     bar = tc_smem(mbar + group);
     phase = 0;
-    dead = false;
+    dead = 0;
     if (threadIdx.x < 32) {
       asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem(tmem_slot)),
                    "n"(512 / kTcCtas)
@@ -410,7 +416,8 @@ struct P2Tc {
     }
     if (threadIdx.x == 0) {
       for (uint32_t g = 0; g < kTcGroups; g++)
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem(mbar + g)) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(tc_smem(mbar + g)), "r"(c_p2_tc[F::ID].arrivals)
+                     : "memory");
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -422,6 +429,9 @@ struct P2Tc {
     grid_wait();
   }
   __device__ __forceinline__ void close() {
+    // A warp that gave up waits once more, as long again: products still in
+    // flight write TMEM columns and a barrier that are about to be given back.
+    if (dead) arrived(dead - 1);
     __syncwarp();
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

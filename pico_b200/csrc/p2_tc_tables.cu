@@ -67,6 +67,8 @@ void build(const uint32_t ext[8][16], const uint32_t* inte, const uint32_t diag[
   B.out = tables;
   memset(tables, 0, kTcTableBytes);
   memset(consts, 0, sizeof *consts);
+  consts->wait_tries = kTcWaitTries;
+  consts->arrivals = 1;
   const uint64_t p = F::P;
   const uint64_t r32inv = [&] {
     uint64_t r = 1, b = B.r32, e = p - 2;

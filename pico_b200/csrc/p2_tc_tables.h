@@ -42,8 +42,11 @@ static_assert(kTcTableBytes % 16 == 0, "operands start on 16 bytes");
 enum TcConstCol : uint32_t { kTcCInit = 0, kTcCMerged = 1, kTcCR1 = 2, kTcCR5 = 5, kTcCOut = 8 };
 
 struct P2TcConstants {
-  int32_t beta[8];  // y of k + 1 rounds ago: Monty form, centred (|.| <= p/2)
+  int32_t beta[8];     // y of k + 1 rounds ago: Monty form, centred (|.| <= p/2)
+  uint32_t wait_tries; // tries of a wait for products before it gives up
+  uint32_t arrivals;   // arrivals that complete a barrier: the products' one (two: no wait ever ends)
 };
+constexpr uint32_t kTcWaitTries = 1u << 18;  // about a second (3.9 us a try)
 
 // Tables of the one-word-per-lane form (p2_lane.cuh), in words; entry [k][i]
 // belongs to lane i.
