@@ -463,10 +463,12 @@ extern "C" pico_status pico_gpu_init(int device, const pico_config* cfg, pico_ct
   }
   {
     void* g = nullptr;
-    const size_t bytes = 2 * ctx->streams.size() * sizeof(GuardRecord);
+    const size_t records = 2 * ctx->streams.size() * sizeof(GuardRecord);
+    const size_t bytes = records + ctx->streams.size() * 4;
     if ((s = cuda_status(cudaMallocHost(&g, bytes), "guard records"))) return s;
     memset(g, 0, bytes);
     ctx->guard_host = (GuardRecord*)g;
+    ctx->permute_expired = (uint32_t*)((uint8_t*)g + records);
     if ((s = cuda_status(lde_guard_clear(), "guard clear")) || (s = cuda_status(hash_guard_clear(), "guard clear")))
       return s;
   }
@@ -580,24 +582,36 @@ pico_status guard_enqueue(pico_ctx* ctx, uint32_t slot, cudaStream_t st) {
   return cuda_status(hash_guard_fetch(ctx->guard_host + 2 * slot + 1, st), "guard read-back");
 }
 
-pico_status guard_verdict(pico_ctx* ctx, uint32_t slot, std::string* msg) {
+std::string guard_message(const GuardRecord* records) {
   static const char* const unit[2] = {"LDE", "row hashing"};
   for (int u = 0; u < 2; u++) {
-    const GuardRecord& g = ctx->guard_host[2 * slot + u];
+    const GuardRecord& g = records[u];
     if (!g.count) continue;
     char buf[256];
-    snprintf(buf, sizeof buf,
-             "internal bounds guard: %s kernel skipped %llu access(es); first: tag %llu, offset %llu of %llu, "
-             "block %llu, thread %llu",
-             unit[u], g.count, g.tag, g.offset, g.extent, g.block, g.thread);
-    if (msg) *msg = buf;
-    set_error("%s", buf);
-    lde_guard_clear();
-    hash_guard_clear();
-    memset(ctx->guard_host + 2 * slot, 0, 2 * sizeof(GuardRecord));
-    return PICO_ERR_CUDA;
+    if (u == 1 && g.tag == kGuardTensorWait)
+      snprintf(buf, sizeof buf,
+               "tensor-core Poseidon2: a wait for a product ran out in %llu thread(s); first: block %llu, thread %llu; "
+               "the results are void",
+               g.count, g.block, g.thread);
+    else
+      snprintf(buf, sizeof buf,
+               "internal bounds guard: %s kernel skipped %llu access(es); first: tag %llu, offset %llu of %llu, "
+               "block %llu, thread %llu",
+               unit[u], g.count, g.tag, g.offset, g.extent, g.block, g.thread);
+    return buf;
   }
-  return PICO_OK;
+  return std::string();
+}
+
+pico_status guard_verdict(pico_ctx* ctx, uint32_t slot, std::string* msg) {
+  const std::string text = guard_message(ctx->guard_host + 2 * slot);
+  if (text.empty()) return PICO_OK;
+  if (msg) *msg = text;
+  set_error("%s", text.c_str());
+  lde_guard_clear();
+  hash_guard_clear();
+  memset(ctx->guard_host + 2 * slot, 0, 2 * sizeof(GuardRecord));
+  return PICO_ERR_CUDA;
 }
 TwiddleTables twiddles(pico_ctx* ctx, int field) {
   TwiddleTables t;
@@ -1746,13 +1760,26 @@ extern "C" pico_status pico_gpu_poseidon2_permute(pico_ctx* ctx, pico_field fiel
   }
   if (!n) return PICO_OK;
   cudaSetDevice(ctx->device);
-  cudaStream_t st = pick_stream(ctx);
+  uint32_t slot = 0;
+  cudaStream_t st = pick_stream(ctx, nullptr, &slot);
   pico_status s;
   const uint64_t bytes = n * 64;
-  if (flags & PICO_INPUT_DEVICE) {
-    if ((s = cuda_status(launch_permute(field, states, n, st, (flags & PICO_P2_FOUR_LANES) != 0), "permute"))) return s;
-    return cuda_status(cudaStreamSynchronize(st), "permute");
-  }
+  const bool four_lanes = (flags & PICO_P2_FOUR_LANES) != 0;
+  // The kernel itself counts waits that ran out, in pinned host memory: a guard
+  // record copied back would cost the call 8-12 us.
+  volatile uint32_t* expired = ctx->permute_expired + slot;
+  const uint32_t expired_before = *expired;
+  auto finish = [&](pico_status r) {
+    const pico_status synced = cuda_status(cudaStreamSynchronize(st), "permute");
+    if (!r) r = synced;
+    if (!r && *expired != expired_before) {
+      set_error("poseidon2_permute: tensor-core Poseidon2: a wait for a product ran out; the results are void");
+      r = PICO_ERR_CUDA;
+    }
+    return r;
+  };
+  if (flags & PICO_INPUT_DEVICE)
+    return finish(cuda_status(launch_permute(field, states, n, st, four_lanes, ctx->permute_expired + slot), "permute"));
   if (!try_reserve(ctx, bytes)) {
     set_error("poseidon2_permute: HBM budget exceeded");
     return PICO_ERR_OUT_OF_MEMORY;
@@ -1760,12 +1787,13 @@ extern "C" pico_status pico_gpu_poseidon2_permute(pico_ctx* ctx, pico_field fiel
   void* d;
   s = alloc_async(&d, bytes, st);
   if (!s) s = cuda_status(cudaMemcpyAsync(d, states, bytes, cudaMemcpyHostToDevice, st), "copy in");
-  if (!s) s = cuda_status(launch_permute(field, (uint32_t*)d, n, st, (flags & PICO_P2_FOUR_LANES) != 0), "permute");
+  if (!s)
+    s = cuda_status(launch_permute(field, (uint32_t*)d, n, st, four_lanes, ctx->permute_expired + slot), "permute");
   if (!s) s = cuda_status(cudaMemcpyAsync(states, d, bytes, cudaMemcpyDeviceToHost, st), "copy out");
   free_async(d, st);
-  pico_status s2 = cuda_status(cudaStreamSynchronize(st), "permute");
+  s = finish(s);
   unreserve(ctx, bytes);
-  return s ? s : s2;
+  return s;
 }
 
 // ---------------------------------------------------------------------------

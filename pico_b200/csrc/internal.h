@@ -74,8 +74,10 @@ constexpr uint64_t kTcMinStates = 1u << 16;
 // traces took 4.78 ms with 2^16, 4.94 with 2^15, 4.49 with 2^14 and 4.39 with
 // 2^13 (runs of one build differ by 0.15 ms, so the last two are equal).
 constexpr uint64_t kTcMinRows = 1u << 13;
-// four_lanes: four threads per state (the latency form).
-cudaError_t launch_permute(int field, uint32_t* states, uint64_t n, cudaStream_t st, bool four_lanes = false);
+// four_lanes: four threads per state (the latency form).  *expired (pinned host
+// memory) changes if a wait of the tensor-core form ran out: states are void.
+cudaError_t launch_permute(int field, uint32_t* states, uint64_t n, cudaStream_t st, bool four_lanes,
+                           uint32_t* expired);
 // At most this many states: 16 lanes per state (p2_lane.cuh).  A FRI phase of
 // 2^23 elements took 4.20 ms with 2^14, 4.11 with this and 4.12 with 2^12.
 constexpr uint64_t kLaneMaxStates = 8192;

@@ -555,7 +555,7 @@ __host__ __device__ static inline uint64_t tc_tiles(uint64_t n) { return (n + kT
   if (tc.dead) hash_guard_trip(0, 0, kGuardTensorWait)
 
 template <class F>
-__global__ void __launch_bounds__(kTcThreads * kTcGroups, kTcCtas) k_permute_tc(uint32_t* states, uint64_t n) {
+__global__ void __launch_bounds__(kTcThreads * kTcGroups, kTcCtas) k_permute_tc(uint32_t* states, uint64_t n, volatile uint32_t* expired) {
   PICO_TC_OPEN(F);
   for (uint64_t t0 = tc.first_tile(tc_tiles(n)) * kTcThreads; t0 < n; t0 += tc.tile_stride() * kTcThreads) {
     const uint64_t i = t0 + threadIdx.x % kTcThreads;
@@ -577,7 +577,8 @@ __global__ void __launch_bounds__(kTcThreads * kTcGroups, kTcCtas) k_permute_tc(
       for (int k = 0; k < 4; k++) p[k] = make_uint4(s[4 * k], s[4 * k + 1], s[4 * k + 2], s[4 * k + 3]);
     }
   }
-  PICO_TC_CLOSE();
+  tc.close();
+  if (tc.dead) *expired = *expired + 1;  // the host looks for any change
 }
 
 // Row digests of a GroupBatch (k_hash_groups' sponges).  Tiles of 128 rows do
@@ -769,7 +770,8 @@ __global__ void __launch_bounds__(256) k_permute_quad(uint32_t* states, uint64_t
   if (live) reinterpret_cast<uint4*>(states + 16 * i)[q] = make_uint4(v[0], v[1], v[2], v[3]);
 }
 
-cudaError_t launch_permute(int field, uint32_t* states, uint64_t n, cudaStream_t st, bool four_lanes) {
+cudaError_t launch_permute(int field, uint32_t* states, uint64_t n, cudaStream_t st, bool four_lanes,
+                           uint32_t* expired) {
   if (n == 0) return cudaSuccess;
   if (four_lanes) {
     if (field == 0)
@@ -780,7 +782,7 @@ cudaError_t launch_permute(int field, uint32_t* states, uint64_t n, cudaStream_t
   }
   if (n >= kTcMinStates) {
     return tc_launch(false, field == 0 ? k_permute_tc<KoalaBear> : k_permute_tc<BabyBear>, tc_tiles(n), false, st, states,
-                     n);
+                     n, expired);
   }
   if (field == 0)
     k_permute<KoalaBear><<<blocks_for(n, 256), 256, 0, st>>>(states, n);

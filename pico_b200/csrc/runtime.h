@@ -98,6 +98,8 @@ pico_status enqueue_fri_rounds(int field, cudaStream_t st, const TwiddleTables& 
                                uint32_t* d_betas, DevChallenger* d_ch, const uint32_t* const* inject,
                                uint32_t* launches = nullptr);
 pico_status guard_enqueue(pico_ctx* ctx, uint32_t slot, cudaStream_t st);
+// What a slot's two host records say, empty if nothing.
+std::string guard_message(const GuardRecord* records);
 pico_status guard_verdict(pico_ctx* ctx, uint32_t slot, std::string* msg = nullptr);
 pico_status finish_stats(pico_commit* c);
 // One JSON line per finished commit or served request into the file named by
@@ -122,6 +124,7 @@ struct pico_ctx {
   std::atomic<uint32_t> next_aux{0};
   uint32_t* tw[2] = {nullptr, nullptr};  // per-field twiddle tables (lo | hi | stage)
   pico::GuardRecord* guard_host = nullptr;  // pinned: 2 records (LDE, hashing) per stream slot
+  uint32_t* permute_expired = nullptr;  // after them, per slot: counts of permute waits that ran out, never reset
   pico::Server* server = nullptr;
   uint32_t max_inflight = 0;  // serving: requests on the device at once
   uint32_t max_group = pico::kDefaultGroup;  // serving: requests admitted together into one slot (shared launches)

@@ -91,11 +91,8 @@ static void CUDART_CB on_request_done(void* arg) {
   // the device records stay set until a synchronous call reports and clears them)
   const GuardRecord* gr = r->ctx->guard_host + 2 * r->slot;
   if (gr[0].count || gr[1].count) {
-    char buf[160];
-    snprintf(buf, sizeof buf, "internal bounds guard: %s kernel skipped an access (tag %llu)",
-             gr[0].count ? "LDE" : "row hashing", gr[0].count ? gr[0].tag : gr[1].tag);
     r->status = PICO_ERR_CUDA;
-    r->error = buf;
+    r->error = guard_message(gr);
   }
   r->t_done = Clock::now();
   r->state = pico_request::DONE;
@@ -166,11 +163,8 @@ static void CUDART_CB on_group_done(void* arg) {
     memcpy(r->root, r->root_pinned, 32);
     memcpy(r->commit->root, r->root_pinned, 32);
     if (gr[0].count || gr[1].count) {
-      char buf[160];
-      snprintf(buf, sizeof buf, "internal bounds guard: %s kernel skipped an access (tag %llu)",
-               gr[0].count ? "LDE" : "row hashing", gr[0].count ? gr[0].tag : gr[1].tag);
       r->status = PICO_ERR_CUDA;
-      r->error = buf;
+      r->error = guard_message(gr);
     }
     r->t_done = done;
     r->state = pico_request::DONE;

@@ -6,7 +6,7 @@ and the context goes on working, the failure not charged to a later call.
 import numpy as np
 import pytest
 
-from pico_b200 import MerkleTreeMmcs, PicoError, TwoAdicFriPcs, abi, new_challenger
+from pico_b200 import MerkleTreeMmcs, PicoError, Poseidon2, TwoAdicFriPcs, abi, new_challenger
 from pico_b200 import fields as F
 
 pytestmark = pytest.mark.gpu
@@ -34,6 +34,7 @@ def _reported(call):
     with pytest.raises(PicoError) as e:
         call()
     assert e.value.status == abi.PICO_ERR_CUDA
+    assert "ran out" in str(e.value)
 
 
 @pytest.mark.parametrize("f", FIELDS)
@@ -63,3 +64,22 @@ def test_fri_commit_phase(gpu, orc, expired, f):
     expired(False)
     got = pcs.fri_commit_phase(_dev(cw), challenger=new_challenger())
     assert (got.roots == want[0]).all() and (got.final_poly == want[2]).all()
+
+
+@pytest.mark.parametrize("f", FIELDS)
+@pytest.mark.parametrize("device", [True, False])
+def test_permutation(gpu, orc, expired, f, device):
+    st = F.to_monty(f, F.uniform(f, 16 * ROWS, 21)).reshape(ROWS, 16)
+    want = orc.permute(f, st)
+    p = Poseidon2(gpu, f)
+    expired(True)
+    _reported(lambda: p.permute(_dev(st) if device else st.copy()))
+    expired(False)
+    # the record is gone: an unrelated call is not charged with it
+    m = F.random_matrix(f, 4, 3, 1)
+    root, pd = MerkleTreeMmcs(gpu, f).commit([m])
+    pd.release()
+    assert (root == orc.mmcs_commit(f, [m])).all()
+    d = _dev(st) if device else st.copy()
+    p.permute(d)
+    assert ((d.cpu().numpy().view(np.uint32) if device else d) == want).all()
