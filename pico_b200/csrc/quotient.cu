@@ -39,6 +39,7 @@ constexpr uint32_t kQExtRegs = 16;
 // Blocks of 64 and 32 threads, which reach further and pack tighter, measured
 // slower: 85 words 202 -> 237 us, 658 words 4.64 ms against 3.25 in the general form.
 constexpr size_t kQStagedSmem = 220 << 10;
+constexpr size_t kQGeneralSmem = (kQBaseRegs + 4 * kQExtRegs) * kQThreads * 4;  // every register in use
 // k_quotient_staged: a base operation whose result is only asserted, the
 // assertion's index in dst.
 constexpr uint32_t kQAssertOf = 32;
@@ -559,7 +560,7 @@ extern "C" pico_status pico_gpu_quotient_values(pico_ctx* ctx, pico_trace_ref pr
       default: break;
     }
   }
-  size_t smem = (size_t)(n_base + 4 * n_ext) * kQThreads * 4;  // at most 64 KiB
+  size_t smem = (size_t)(n_base + 4 * n_ext) * kQThreads * 4;  // at most kQGeneralSmem
   const StagedProgram sp(program, n_ops, public_values, global_sum);
   const size_t staged_smem = (size_t)sp.stride * kQThreads * 4;
   const bool staged = staged_smem <= kQStagedSmem;
@@ -629,7 +630,10 @@ extern "C" pico_status pico_gpu_quotient_values(pico_ctx* ctx, pico_trace_ref pr
     void (*const kernel)(QuotientArgs, TwiddleTables) =
         field == PICO_KOALABEAR ? (staged ? k_quotient_staged<KoalaBear> : k_quotient<KoalaBear>)
                                 : (staged ? k_quotient_staged<BabyBear> : k_quotient<BabyBear>);
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // the form's maximum and not this program's size: the attribute is the
+    // process's, and another thread may set it between here and the launch
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)(staged ? kQStagedSmem : kQGeneralSmem));
     if (!e) kernel<<<grid, kQThreads, smem, st>>>(A, tw);
     s = cuda_status(e ? e : cudaGetLastError(), "quotient kernel");
   }
