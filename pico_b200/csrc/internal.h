@@ -5,17 +5,11 @@
 
 #include <cstdint>
 
+#include "row_cursor.cuh"
+
 namespace pico {
 
 constexpr int kMaxSegs = 64;  // matrices concatenated into one Merkle row
-
-// One matrix segment of a concatenated Merkle row: `rows` x `width`,
-// row-major, rows at ptr + r * width.
-struct RowSeg {
-  const uint32_t* ptr;
-  uint32_t width;
-  uint32_t pad;
-};
 
 // Rows of all matrices of one height, concatenated in commit order (the
 // MerkleTreeMmcs leaf / injection input, fri.rs:389-436).

@@ -87,6 +87,10 @@ __device__ __forceinline__ void hash_guard_trip(unsigned long long seg, unsigned
     g_hash_guard.thread = threadIdx.x;
   }
 }
+// For row_chunk: a read past the last segment.
+struct RowReadTrip {
+  __device__ __forceinline__ void operator()(uint32_t seg, uint32_t col) const { hash_guard_trip(seg, col); }
+};
 template <class F>
 __device__ __forceinline__ void hash_row_segs(const RowSeg* segs, uint32_t n_segs, uint32_t W, uint64_t r,
                                               uint32_t s[16]) {
@@ -504,45 +508,6 @@ __global__ void k_challenger_observe(DevChallenger* ch, const uint32_t* vals, ui
 // Tensor-core forms (p2_tc.cuh): 128 states per CTA of 128 threads, four CTAs
 // per SM (their 4 x 128 TMEM columns).
 
-// The next up to 8 columns of row r: words of chunk positions [lo, hi) into
-// v, through the segment cursor (seg, col, segw, rowp).
-struct RowCursor {
-  uint32_t seg, col, segw;
-  const uint32_t* rowp;
-};
-__device__ __forceinline__ void row_cursor_begin(RowCursor& c, const RowSeg* segs, uint32_t n_segs, uint64_t r) {
-  c.seg = c.col = 0;
-  c.segw = n_segs ? segs[0].width : 0u;
-  c.rowp = n_segs ? segs[0].ptr + r * c.segw : nullptr;
-}
-__device__ __forceinline__ void row_chunk(RowCursor& c, const RowSeg* segs, uint32_t n_segs, uint64_t r, int lo, int hi,
-                                          uint32_t v[8]) {
-  if (lo == 0 && hi == 8 && c.segw - c.col >= 8) {
-#pragma unroll
-    for (int j = 0; j < 8; j++) v[j] = __ldg(c.rowp + c.col + j);
-    c.col += 8;
-    return;
-  }
-#pragma unroll
-  for (int j = 0; j < 8; j++) {
-    if (j >= lo && j < hi) {
-      while (c.col == c.segw && c.seg < n_segs) {
-        c.seg++;
-        c.col = 0;
-        c.segw = c.seg < n_segs ? segs[c.seg].width : 0u;
-        c.rowp = c.seg < n_segs ? segs[c.seg].ptr + r * c.segw : nullptr;
-      }
-      if (c.seg >= n_segs) {
-        hash_guard_trip(c.seg, c.col);
-        v[j] = 0;
-      } else {
-        v[j] = __ldg(c.rowp + c.col);
-      }
-      c.col++;
-    }
-  }
-}
-
 __host__ __device__ static inline uint64_t tc_tiles(uint64_t n) { return (n + kTcThreads - 1) / kTcThreads; }
 #define PICO_TC_OPEN(F)                                  \
   extern __shared__ __align__(128) uint8_t tc_tables[];  \
@@ -617,7 +582,7 @@ __global__ void __launch_bounds__(kTcThreads * kTcGroups, kTcCtas) k_hash_groups
           tc.output(s);
           from = kTcFromState;
         }
-        row_chunk(cur, segs, s1 - s0, rr, 0, hi, s);
+        row_chunk(cur, segs, s1 - s0, rr, 0, hi, s, RowReadTrip());
         if (from == kTcFromState)
           tc.put_state(s);
         else
@@ -667,7 +632,7 @@ __global__ void __launch_bounds__(kTcThreads * kTcGroups, kTcCtas)
         tc.output(s);
         held = true;
       }
-      row_chunk(cur, g.segs, g.n_segs, rr, lo, hi, s);
+      row_chunk(cur, g.segs, g.n_segs, rr, lo, hi, s, RowReadTrip());
       if (!permute) break;
       if (held)
         tc.put_state(s);
