@@ -29,7 +29,7 @@ cudaError_t upload_p2_constants(int field, const uint32_t ext[8][16], const uint
   std::vector<uint8_t> tables(kTcTableBytes);
   P2TcConstants tc;
   std::vector<uint32_t> lane(kLaneWords);
-  build_p2_tc_tables(field, h.ext, h.inte, h.diag, tables.data(), &tc, lane.data());
+  if (!build_p2_tc_tables(field, h.ext, h.inte, h.diag, tables.data(), &tc, lane.data())) return cudaErrorInvalidValue;
   if ((e = cudaMemcpyToSymbol(g_p2_lane, lane.data(), kLaneWords * 4, (size_t)kLaneWords * 4 * (field ? 1 : 0)))) return e;
   if ((e = cudaMemcpyToSymbol(g_p2_tc, tables.data(), kTcTableBytes, (size_t)kTcTableBytes * (field ? 1 : 0)))) return e;
   return cudaMemcpyToSymbol(c_p2_tc, &tc, sizeof tc, sizeof tc * (field ? 1 : 0));

@@ -215,8 +215,8 @@ struct P2Tc {
   // An output word from its limbs: V = l0 + 2^8 l1 + 2^16 l2 + 2^24 l3 times
   // 2^-16 (the tables carry the 2^16), by one 16-bit Montgomery step:
   // p = 1 mod 2^16, so V - (V mod 2^16) p is divisible by 2^16.  The
-  // constants' top byte is at most 0x7f, so the result lies in
-  // (-p, 1.3e9), and below p/3 where K is one state.
+  // result lies in (-p, p), which the S-boxes and canon() take: the table
+  // builder checks the upper end (at most 8.8e8 with these tables).
   static __device__ __forceinline__ uint32_t recombine(const uint32_t* l) {
     const uint32_t s01 = l[0] + (l[1] << 8), s23 = l[2] + (l[3] << 8);
     return s23 + (s01 >> 16) - (s01 & 0xffffu) * ((F::P - 1) >> 16);
@@ -268,7 +268,9 @@ struct P2Tc {
     tc_st16(lane + kTcZ + 16, z);
   }
   // One block of R partial rounds: inputs from the accumulators plus the
-  // block's own y, which go to K step k.
+  // block's own y, which go to K step k.  Up to kTcBlock - 1 signed products are
+  // added before the fold: with these fields' beta (beta_0 is -1 times 2^32) at
+  // most 0.47 of 2^63 (p2_tc_sums_fit; six of p / 2 each would not fit).
   // Round r's input before the S-box is (X_r + sum_k beta_k y_(r-1-k)) 2^-32.
   template <int R>
   __device__ __forceinline__ void partial_block(uint32_t k) {

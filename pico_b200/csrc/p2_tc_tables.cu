@@ -3,6 +3,7 @@
 // round constants and the internal diagonal.  Plain 64-bit integer arithmetic
 // on canonical values.
 #include <cstring>
+#include <initializer_list>
 #include <vector>
 
 #include "field.cuh"
@@ -55,10 +56,39 @@ struct Builder {
       out[col + (n / 8) * 128 + (n % 8) * 16 + 12] = (uint8_t)(v >> (8 * l));
     }
   }
+  // The recombined outputs of a stage: `outputs` of them, from K steps of these
+  // tables and a constant column (or 0).
+  struct Part {
+    uint32_t table, steps;
+  };
+  bool limbs_fit(uint32_t N, uint32_t outputs, std::initializer_list<Part> parts, uint32_t col) const {
+    for (uint32_t i = 0; i < outputs; i++) {
+      uint64_t limb[4] = {0, 0, 0, 0};
+      for (uint32_t l = 0; l < 4; l++) {
+        for (const Part& part : parts)
+          for (uint32_t s = 0; s < part.steps; s++)
+            for (uint32_t k = 0; k < 32; k++) limb[l] += 255u * out[part.table + s * N * 32 + at(N, 4 * i + l, k)];
+        const uint32_t n = 4 * i + l;
+        if (col) limb[l] += out[col + (n / 8) * 128 + (n % 8) * 16 + 12];
+      }
+      if (limb[0] + (limb[1] << 8) >= (1ull << 32) || limb[2] + (limb[3] << 8) + 65535 >= p) return false;
+    }
+    return true;
+  }
+  bool all_limbs_fit(int rounds_p) const {
+    const uint32_t y_steps = rounds_p > 2 * kTcBlock ? 3 : 2;  // of the state after the partial rounds
+    bool fit = limbs_fit(64, 16, {{kTcFull, 4}}, kTcC + 1024 * kTcCInit) &&
+               limbs_fit(64, 16, {{kTcNew, 1}}, kTcC + 1024 * kTcCInit) &&
+               limbs_fit(64, 16, {{kTcE2, 4}, {kTcNew, 1}}, kTcC + 1024 * kTcCMerged) &&
+               limbs_fit(32, kTcBlock, {{kTcP1, 4}}, kTcCP1) && limbs_fit(32, kTcBlock, {{kTcP2, 5}}, 0) &&
+               limbs_fit(32, kTcBlock, {{kTcP3, 6}}, 0) && limbs_fit(64, 16, {{kTcFin, 4 + y_steps}}, 0);
+    for (uint32_t c = kTcCR1; c <= kTcCOut; c++) fit = fit && limbs_fit(64, 16, {{kTcFull, 4}}, kTcC + 1024 * c);
+    return fit;
+  }
 };
 
 template <class F>
-void build(const uint32_t ext[8][16], const uint32_t* inte, const uint32_t diag[16], uint8_t* tables,
+bool build(const uint32_t ext[8][16], const uint32_t* inte, const uint32_t diag[16], uint8_t* tables,
            P2TcConstants* consts, uint32_t* lane) {
   constexpr int R = F::ROUNDS_P;
   Builder B;
@@ -194,16 +224,22 @@ void build(const uint32_t ext[8][16], const uint32_t* inte, const uint32_t diag[
     lane[kLaneConst + 32 + i] = monty(ext[4][i]);
   }
   for (int k = 0; k < R; k++) lane[kLaneBeta + kLaneBetaZero + k] = monty(beta[k]);
+  return p2_tc_sums_fit(consts->beta, F::P) && B.all_limbs_fit(R);
 }
 
 }  // namespace
 
-void build_p2_tc_tables(int field, const uint32_t ext[8][16], const uint32_t* inte, const uint32_t diag[16],
+bool p2_tc_sums_fit(const int32_t beta[8], uint32_t p) {
+  uint64_t sum = 0;
+  for (int k = 0; k < kTcBlock - 1; k++) sum += beta[k] < 0 ? 0u - (uint32_t)beta[k] : (uint32_t)beta[k];
+  const uint64_t y = 3ull * p / 4;
+  return sum <= ((1ull << 63) - 1 - p) / y;
+}
+
+bool build_p2_tc_tables(int field, const uint32_t ext[8][16], const uint32_t* inte, const uint32_t diag[16],
                         uint8_t* tables, P2TcConstants* consts, uint32_t* lane) {
-  if (field == 0)
-    build<KoalaBear>(ext, inte, diag, tables, consts, lane);
-  else
-    build<BabyBear>(ext, inte, diag, tables, consts, lane);
+  return field == 0 ? build<KoalaBear>(ext, inte, diag, tables, consts, lane)
+                    : build<BabyBear>(ext, inte, diag, tables, consts, lane);
 }
 
 }  // namespace pico

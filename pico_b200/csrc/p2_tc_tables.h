@@ -60,9 +60,20 @@ constexpr uint32_t kLaneBetaZero = 24;
 constexpr uint32_t kLaneWords = kLaneBeta + 64;
 static_assert(kLaneWords % 4 == 0, "copied by 16 bytes");
 
+// Whether the sums a block of partial rounds forms stay inside 63 bits: its last
+// round adds kTcBlock - 1 products beta_k y and one recombined word.  The word is
+// at most p.  |y| is below 3 p / 4: the S-box input is within p / 2 + 2^28 (the
+// sum's high word is folded by 2^32 mod p < 2^29 before the reduction), below
+// 0.64 p in both fields, and each product of factors below f p and g p reduces to
+// (f g r + 1/2) p, r = p / 2^32, which gives 0.72 p (x^3) and 0.74 p (x^7).
+bool p2_tc_sums_fit(const int32_t beta[8], uint32_t p);
 // The tables of one field (kTcTableBytes) and its multiply-accumulate
-// constants, and the lane tables (kLaneWords), from the canonical round constants and diagonal.
-void build_p2_tc_tables(int field, const uint32_t ext[8][16], const uint32_t* inte, const uint32_t diag[16],
+// constants, and the lane tables (kLaneWords), from the canonical round constants
+// and diagonal.  False if with these some sum of the tensor-core form could leave
+// its range: those of p2_tc_sums_fit, or, with every byte 255, the limbs of an
+// output (l0 + 2^8 l1 in 32 bits, and l2 + 2^8 l3, the recombined word's upper
+// end, below p).
+bool build_p2_tc_tables(int field, const uint32_t ext[8][16], const uint32_t* inte, const uint32_t diag[16],
                         uint8_t* tables, P2TcConstants* consts, uint32_t* lane);
 
 }  // namespace pico
