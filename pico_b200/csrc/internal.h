@@ -75,7 +75,8 @@ cudaError_t launch_permute(int field, uint32_t* states, uint64_t n, cudaStream_t
 // At most this many states: 16 lanes per state (p2_lane.cuh).  A FRI phase of
 // 2^23 elements took 4.20 ms with 2^14, 4.11 with this and 4.12 with 2^12.
 constexpr uint64_t kLaneMaxStates = 8192;
-// Levels of at most this many nodes are compressed four threads per node.
+// Levels of at most this many nodes are compressed four threads per node (in a
+// tree, the one of 2^14: k_subtree_lane makes the narrower ones).
 constexpr uint64_t kQuadMaxNodes = 16384;
 cudaError_t launch_hash_rows(int field, const RowGroup& g, uint64_t rows, uint32_t* out, cudaStream_t st,
                              unsigned block = 256);
@@ -119,6 +120,7 @@ cudaError_t launch_subtree(int field, uint32_t* level, uint32_t n_in, uint32_t n
 // at most 32 nodes to make (two per warp), twice that at 64.
 constexpr uint32_t kSubtreeMaxLog = 14;
 inline uint32_t subtree_log_in(uint32_t log_n) { return log_n <= 7 ? log_n : log_n <= 13 ? log_n - 6 : 7; }
+// One level of a tree wider than k_subtree_lane takes:
 // next[i] = compress(prev[2i], prev[2i+1]); if inj_digests != null:
 // next[i] = compress(next[i], inj_digests[i]) (8 words per digest).
 cudaError_t launch_compress(int field, const uint32_t* prev, uint32_t* next, uint64_t n_next,

@@ -276,27 +276,6 @@ __global__ void __launch_bounds__(256)
 // rows too few to fill the GPU.
 constexpr uint32_t kLaneThreads = 256;  // 16 states per CTA
 
-template <class F>
-__global__ void __launch_bounds__(kLaneThreads) k_compress_lane(const uint32_t* prev, uint32_t* next, uint64_t n,
-                                                                const uint32_t* inj) {
-  __shared__ __align__(16) uint32_t tab[kLaneWords];
-  lane_load_tables<F>(tab);
-  const uint64_t t = blockIdx.x * (uint64_t)kLaneThreads + threadIdx.x;
-  const uint64_t i = t >> 4;
-  const uint32_t q = (uint32_t)(t & 15);
-  const bool live = i < n;
-  uint32_t v = live ? prev[16 * i + q] : 0u;
-  uint32_t d = 0;
-  if (inj && live && q >= 8) d = inj[8 * i + q - 8];
-  __syncthreads();
-  v = lane_permute<F>(v, q, tab);
-  if (inj) {
-    if (q >= 8) v = d;
-    v = lane_permute<F>(v, q, tab);
-  }
-  if (live && q < 8) next[8 * i + q] = v;
-}
-
 // Row digests of a GroupBatch, 16 lanes per row (k_hash_groups' sponges): lanes
 // 0..7 carry the rate, so a chunk's eight words are one load.
 template <class F>
@@ -848,8 +827,8 @@ cudaError_t launch_absorb_rows(int field, const RowGroup& g, uint64_t rows, uint
   return cudaGetLastError();
 }
 
-// The same compression, four threads per node (levels too small to fill the
-// GPU, where one permutation's latency sets the launch's time).
+// The same compression, four threads per node (the level of 2^14 nodes, too few
+// to fill the GPU: one permutation's latency sets the launch's time).
 template <class F>
 __global__ void __launch_bounds__(256) k_compress_quad(const uint32_t* prev, uint32_t* next, uint64_t n,
                                                        const uint32_t* inj) {
@@ -881,10 +860,6 @@ __global__ void __launch_bounds__(256) k_compress_quad(const uint32_t* prev, uin
 cudaError_t launch_compress(int field, const uint32_t* prev, uint32_t* next, uint64_t n_next,
                             const uint32_t* inj_digests, cudaStream_t st, bool chained) {
   if (n_next == 0) return cudaSuccess;
-  if (n_next <= kLaneMaxStates) {
-    return launch_chained(chained, field == 0 ? k_compress_lane<KoalaBear> : k_compress_lane<BabyBear>,
-                          blocks_for(16 * n_next, kLaneThreads), kLaneThreads, 0, st, prev, next, n_next, inj_digests);
-  }
   if (n_next <= kQuadMaxNodes) {
     if (field == 0)
       k_compress_quad<KoalaBear><<<blocks_for(4 * n_next, 256), 256, 0, st>>>(prev, next, n_next, inj_digests);
