@@ -8,12 +8,11 @@
 // point i + 2^log_qd (mod Q).  The chip's constraints come as a straight-line
 // register program (pico_constraint_op, see include/pico_gpu.h) that every
 // thread runs over its own registers, which live in shared memory, in one of
-// two forms: k_quotient_staged, and k_quotient for programs that read too many
-// words.  Assertions fold as acc = acc * alpha + c
+// two forms, k_quotient_staged or k_quotient, by what the program reads and does
+// (ProgramShape, quotient_program.h).  Assertions fold as acc = acc * alpha + c
 // (ProverConstraintFolder::assert_zero / assert_zero_ext,
-// vm/src/machine/folder.rs:223-227,321-327), computed as the sum of
-// alpha^(m-1-k) c_k over the m assertions; the quotient is acc * inv_zerofier.  The Lagrange selectors for the trace domain
-// H = <w_n> (shift 1) follow vm/src/compiler/recursion/circuit/domain.rs:48-66:
+// vm/src/machine/folder.rs:223-227,321-327); the quotient is acc * inv_zerofier.
+// The Lagrange selectors for the trace domain H = <w_n> (shift 1) follow vm/src/compiler/recursion/circuit/domain.rs:48-66:
 // Z_H(x) = x^n - 1, is_first_row = Z_H / (x - 1), is_last_row =
 // Z_H / (x - w_n^-1), is_transition = x - w_n^-1, inv_zerofier = 1 / Z_H; the
 // three inverses share one Fermat inversion per point.
@@ -26,29 +25,25 @@
 #include "../../include/pico_gpu.h"
 #include "field.cuh"
 #include "internal.h"
+#include "quotient_program.h"
 #include "runtime.h"
 
 namespace pico {
 
-constexpr int kQThreads = 128;
 constexpr uint32_t kQBaseRegs = 64;  // register file limits of a program
 constexpr uint32_t kQExtRegs = 16;
-// Shared memory per CTA up to which a program runs in the staged form: it is
-// faster down to one CTA per SM.  2^18 points of a program that reads 149 / 202 /
-// 311 words: 497 / 770 / 2,000 us, in the general form 696 / 1,364 / 3,000.
-// Blocks of 64 and 32 threads, which reach further and pack tighter, measured
-// slower: 85 words 202 -> 237 us, 658 words 4.64 ms against 3.25 in the general form.
-constexpr size_t kQStagedSmem = 220 << 10;
 constexpr size_t kQGeneralSmem = (kQBaseRegs + 4 * kQExtRegs) * kQThreads * 4;  // every register in use
 // k_quotient_staged: a base operation whose result is only asserted, the
 // assertion's index in dst.
 constexpr uint32_t kQAssertOf = 32;
 
-// Sum of power * value over the assertions, one 64-bit sum per coefficient,
-// its high word kept below p (p^2 + p 2^32 < 2^64).  A base value costs four
-// wide multiply-adds and eight additions; the product acc * alpha it stands
-// for is 19 Montgomery products: 2^20 points, 32 assertions in 215
-// instructions, 605 -> 579 us (the column reads bound the rest).
+// The fold in the staged form: the sum of alpha^(m-1-k) c_k over the m
+// assertions, one 64-bit sum per coefficient, its high word kept below p (p^2 +
+// p 2^32 < 2^64).  A base value costs four wide multiply-adds and eight
+// additions; the product acc * alpha it stands for is 19 Montgomery products.
+// The general form folds as written: there the powers are one more read per
+// assertion that the column reads push out of the L1 (2^18 points, 300 columns and
+// assertions 2,290 us, with the sum 3,010; 2^20 points, 200 columns 7.7 / 9.4 ms).
 template <class F>
 struct AssertSum {
   uint32_t lo[4] = {0, 0, 0, 0}, hi[4] = {0, 0, 0, 0};
@@ -65,8 +60,11 @@ struct AssertSum {
 #pragma unroll
     for (int j = 0; j < 4; j++) hi[j] = Fp<F>::add(hi[j], v.c[j]);
   }
-  __device__ __forceinline__ uint32_t value(int j) const {
-    return Fp<F>::canon(Fp<F>::redc(((uint64_t)hi[j] << 32) | lo[j]));
+  __device__ __forceinline__ Ext4 value() const {
+    Ext4 v;
+#pragma unroll
+    for (int j = 0; j < 4; j++) v.c[j] = Fp<F>::canon(Fp<F>::redc(((uint64_t)hi[j] << 32) | lo[j]));
+    return v;
   }
 };
 
@@ -77,7 +75,8 @@ struct QuotientArgs {
   uint32_t main_w, prep_w, perm_w;  // words per row (perm: 4 per extension column)
   const uint4* ops;
   uint32_t n_ops;
-  const uint4* powers;      // alpha^(m-1-k) for the k-th of m assertions, whose dst is k
+  uint32_t alpha[4];
+  const uint4* powers;      // k_quotient_staged: alpha^(m-1-k) for the k-th of m assertions, whose dst is k
   const uint32_t* pub;      // public values
   const uint32_t* chal;     // permutation challenges, 4 words each
   const uint32_t* consts;   // regional sum (4), global sum (14)
@@ -137,13 +136,12 @@ __device__ __forceinline__ Selectors selectors(uint64_t i, const QuotientArgs& A
   return {B::mul(zh, B::mul(d2, zi)), B::mul(zh, B::mul(d1, zi)), d2, B::mul(inv, d12)};
 }
 template <class F>
-__device__ __forceinline__ void store_quotient(const AssertSum<F>& acc, uint32_t inv_zh, uint64_t i,
-                                               const QuotientArgs& A) {
+__device__ __forceinline__ void store_quotient(const Ext4& acc, uint32_t inv_zh, uint64_t i, const QuotientArgs& A) {
   using B = Fp<F>;
   const uint64_t orow =
       A.chunks ? ((i & ((1ull << A.log_qd) - 1)) << A.log_trace) + (i >> A.log_qd) : i;  // a permutation of [0, Q)
-  reinterpret_cast<uint4*>(A.out)[orow] = make_uint4(B::mul(acc.value(0), inv_zh), B::mul(acc.value(1), inv_zh),
-                                                     B::mul(acc.value(2), inv_zh), B::mul(acc.value(3), inv_zh));
+  reinterpret_cast<uint4*>(A.out)[orow] = make_uint4(B::mul(acc.c[0], inv_zh), B::mul(acc.c[1], inv_zh),
+                                                     B::mul(acc.c[2], inv_zh), B::mul(acc.c[3], inv_zh));
 }
 
 template <class F>
@@ -163,7 +161,8 @@ __global__ void __launch_bounds__(kQThreads) k_quotient(const __grid_constant__ 
   const uint64_t row_n = bitrev64((ii + (1ull << A.log_qd)) & (Q - 1), (int)log_q);
 
   const Selectors sel = selectors<F>(ii, A, tw);
-  AssertSum<F> acc;
+  Ext4 acc{{0, 0, 0, 0}};
+  const Ext4 alpha{{A.alpha[0], A.alpha[1], A.alpha[2], A.alpha[3]}};
 
   auto ext_get = [&](uint32_t r) {
     Ext4 v;
@@ -208,15 +207,19 @@ __global__ void __launch_bounds__(kQThreads) k_quotient(const __grid_constant__ 
         ext_set(d, Ext4{{__ldg(A.consts), __ldg(A.consts + 1), __ldg(A.consts + 2), __ldg(A.consts + 3)}});
         break;
       case PICO_Q_GLOBAL: rb[d * kQThreads] = __ldg(A.consts + 4 + a); break;
-      case PICO_Q_ASSERT: acc.add_base(__ldg(A.powers + d), rb[a * kQThreads]); break;
-      case PICO_Q_EASSERT: acc.add_ext(__ldg(A.powers + d), ext_get(a)); break;
+      case PICO_Q_ASSERT: {
+        acc = E::mul(acc, alpha);
+        acc.c[0] = B::add(acc.c[0], rb[a * kQThreads]);
+        break;
+      }
+      case PICO_Q_EASSERT: acc = E::add(E::mul(acc, alpha), ext_get(a)); break;
       default: break;  // validated on the host
     }
   }
-  if (active) store_quotient(acc, sel.inv_zh, i, A);
+  if (active) store_quotient<F>(acc, sel.inv_zh, i, A);
 }
 
-// The staged form, where a point's words fit in shared memory: thread t of CTA b
+// The staged form: thread t of CTA b
 // owns the point of committed row 128 b + t and a row of shared memory
 // that holds the trace words the program reads (each copied once, a row's
 // words side by side), the selectors and the program's registers; the odd
@@ -305,7 +308,7 @@ __global__ void __launch_bounds__(kQThreads) k_quotient_staged(const __grid_cons
     }
     o = following;
   }
-  if (active) store_quotient(acc, sel.inv_zh, i, A);
+  if (active) store_quotient<F>(acc.value(), sel.inv_zh, i, A);
 }
 
 }  // namespace pico
@@ -336,9 +339,9 @@ void assertion_powers(const uint32_t alpha[4], uint32_t m, uint32_t* powers) {
 // words of their own) and public values and global sums are constants.
 struct StagedProgram {
   std::vector<uint32_t> cols;
-  uint32_t cols_end[6];
+  uint32_t cols_end[6] = {};
   std::vector<pico_constraint_op> ops;
-  uint32_t stride;
+  uint32_t stride = 1;
   // For each assertion of a base register: its value comes from the addition,
   // subtraction or product just before it, and nothing reads that register
   // again before it is written.
@@ -368,24 +371,21 @@ struct StagedProgram {
     }
     return sole;
   }
-  StagedProgram(const pico_constraint_op* program, uint32_t n_ops, const uint32_t* public_values,
-                const uint32_t* global_sum) {
-    auto list = [](const pico_constraint_op& o) {
-      return (o.op == PICO_Q_MAIN ? 0u : o.op == PICO_Q_PREP ? 2u : 4u) + o.b;
-    };
-    auto reads = [](const pico_constraint_op& o) {
-      return o.op == PICO_Q_MAIN || o.op == PICO_Q_PREP || o.op == PICO_Q_PERM;
-    };
-    std::vector<uint32_t> used[6];
-    for (uint32_t k = 0; k < n_ops; k++)
-      if (reads(program[k])) used[list(program[k])].push_back(program[k].a);
+  StagedProgram() = default;
+  StagedProgram(const pico_constraint_op* program, uint32_t n_ops, const ProgramShape& shape,
+                const uint32_t* public_values, const uint32_t* global_sum) {
+    std::vector<uint32_t> word[6];  // per column of a list, its (first) word
+    cols.reserve(shape.words);
     for (uint32_t l = 0; l < 6; l++) {
-      std::sort(used[l].begin(), used[l].end());
-      used[l].erase(std::unique(used[l].begin(), used[l].end()), used[l].end());
-      for (uint32_t c : used[l])
+      word[l].assign(shape.last[l].size(), 0);
+      for (uint32_t c = 0; c < word[l].size(); c++) {
+        if (!shape.last[l][c]) continue;
+        word[l][c] = (uint32_t)cols.size();
         for (uint32_t j = 0; j < (l < 4 ? 1u : 4u); j++) cols.push_back(l < 4 ? c : 4 * c + j);
+      }
       cols_end[l] = (uint32_t)cols.size();
     }
+    ops.reserve(n_ops + 1);
     const uint32_t selectors = (uint32_t)cols.size();
     uint32_t words = selectors + 3;
     constexpr uint32_t kNone = 0xffffffffu;
@@ -410,8 +410,8 @@ struct StagedProgram {
       pico_constraint_op o = program[k];
       switch (o.op) {
         case PICO_Q_MAIN: case PICO_Q_PREP: case PICO_Q_PERM: {
-          const uint32_t l = list(o), at = (uint32_t)(std::lower_bound(used[l].begin(), used[l].end(), o.a) - used[l].begin());
-          now[l < 4 ? 0 : 1][o.dst] = (l ? cols_end[l - 1] : 0u) + (l < 4 ? at : 4 * at);
+          const int l = ProgramShape::list(o);
+          now[l < 4 ? 0 : 1][o.dst] = word[l][o.a];
           continue;
         }
         case PICO_Q_FIRST: case PICO_Q_LAST: case PICO_Q_TRANSITION:
@@ -561,13 +561,15 @@ extern "C" pico_status pico_gpu_quotient_values(pico_ctx* ctx, pico_trace_ref pr
     }
   }
   size_t smem = (size_t)(n_base + 4 * n_ext) * kQThreads * 4;  // at most kQGeneralSmem
-  const StagedProgram sp(program, n_ops, public_values, global_sum);
-  const size_t staged_smem = (size_t)sp.stride * kQThreads * 4;
-  const bool staged = staged_smem <= kQStagedSmem;
   const uint64_t Q = 1ull << log_q;
+  const unsigned grid = (unsigned)((Q + kQThreads - 1) / kQThreads);
+  const ProgramShape shape(program, n_ops, wm, wp, we / 4);
+  const bool staged = shape.prefer_staged(shape.words + 3 + n_base + 4 * n_ext, grid, 4 * Q * ((uint64_t)wm + wp + we),
+                                          (uint32_t)ctx->sm_count);
+  const StagedProgram sp = staged ? StagedProgram(program, n_ops, shape, public_values, global_sum) : StagedProgram();
   const bool out_dev = flags & PICO_OUTPUT_DEVICE;
   // one device block: program, assertion powers, public values, challenges, constants, then the output if on the host
-  const uint64_t w_ops = 4ull * (staged ? sp.ops.size() : n_ops), w_pow = 4ull * n_asserts, w_pub = n_public, w_chal = 4ull * n_challenges;
+  const uint64_t w_ops = 4ull * (staged ? sp.ops.size() : n_ops), w_pow = staged ? 4ull * n_asserts : 0, w_pub = n_public, w_chal = 4ull * n_challenges;
   const uint64_t w_const = 18;
   const uint64_t o_pub = w_ops + w_pow, o_chal = o_pub + w_pub, o_const = o_chal + w_chal, o_cols = o_const + w_const;
   const uint64_t w_in = o_cols + (staged ? sp.cols.size() : 0);
@@ -588,14 +590,12 @@ extern "C" pico_status pico_gpu_quotient_values(pico_ctx* ctx, pico_trace_ref pr
   if (staged) {
     memcpy(host.data(), sp.ops.data(), 4 * w_ops);
     if (!sp.cols.empty()) memcpy(host.data() + o_cols, sp.cols.data(), 4 * sp.cols.size());
-    smem = staged_smem;
+    smem = (size_t)sp.stride * kQThreads * 4;
+    if (field == PICO_KOALABEAR) assertion_powers<KoalaBear>(alpha, n_asserts, host.data() + w_ops);
+    else assertion_powers<BabyBear>(alpha, n_asserts, host.data() + w_ops);
   } else {
     if (n_ops) memcpy(host.data(), program, 16ull * n_ops);
-    for (uint32_t k = 0, m = 0; k < n_ops; k++)
-      if (program[k].op == PICO_Q_ASSERT || program[k].op == PICO_Q_EASSERT) host[4ull * k + 1] = m++;
   }
-  if (field == PICO_KOALABEAR) assertion_powers<KoalaBear>(alpha, n_asserts, host.data() + w_ops);
-  else assertion_powers<BabyBear>(alpha, n_asserts, host.data() + w_ops);
   if (n_public) memcpy(host.data() + o_pub, public_values, 4ull * n_public);
   if (n_challenges) memcpy(host.data() + o_chal, perm_challenges, 16ull * n_challenges);
   uint32_t* cst = host.data() + o_const;
@@ -618,6 +618,7 @@ extern "C" pico_status pico_gpu_quotient_values(pico_ctx* ctx, pico_trace_ref pr
   A.log_trace = log_trace_height;
   A.log_qd = log_quotient_degree;
   A.n_base = n_base;
+  memcpy(A.alpha, alpha, 16);
   A.shift_n = field == PICO_KOALABEAR ? shift_power<KoalaBear>(log_trace_height) : shift_power<BabyBear>(log_trace_height);
   A.stride = sp.stride;
   memcpy(A.cols_end, sp.cols_end, sizeof(A.cols_end));
@@ -625,7 +626,6 @@ extern "C" pico_status pico_gpu_quotient_values(pico_ctx* ctx, pico_trace_ref pr
   A.chunks = (flags & PICO_QUOTIENT_CHUNKS) ? 1u : 0u;
   A.out = out_dev ? out : blk + off_out;
   const TwiddleTables tw = twiddles(ctx, field);
-  const unsigned grid = (unsigned)((Q + kQThreads - 1) / kQThreads);
   if (!s) {
     void (*const kernel)(QuotientArgs, TwiddleTables) =
         field == PICO_KOALABEAR ? (staged ? k_quotient_staged<KoalaBear> : k_quotient<KoalaBear>)
