@@ -153,8 +153,9 @@ IMAD_PER_MODMUL = 4
 IMAD_PER_SM_CLK = 64
 # DRAM bytes per algorithmic byte of one leaf-hashing launch (dram__bytes_read
 # + dram__bytes_write over rows * (4 * width + 32)), from an ncu capture of
-# k_hash_rows on a 2^23-row x 16-column LDE (the single-kb-2^22x16 workload)
-HASH_TRAFFIC_RATIO = 0.966
+# k_hash_groups_tc on a 2^23-row x 16-column LDE (the single-kb-2^22x16 workload):
+# 537.0 MB read, 244.5 MB written
+HASH_TRAFFIC_RATIO = 781.6 / 805.3
 # DRAM bytes per algorithmic byte (input + output) of one three-pass LDE, from
 # an ncu capture of k_lde_a/b/c on a 2^22 x 16 matrix at split 2^11 x 2^11:
 # 2,305 MB (read + write over the three passes) for 805 MB algorithmic.  The

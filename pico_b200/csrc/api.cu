@@ -1103,8 +1103,10 @@ struct HashBatcher {
 };
 
 // Commits of at most this many trace cells launch all their LDEs together;
-// above, the tallest group's runs just before its rows are hashed (all
-// together, 48 BabyBear traces of 2^30.9 cells took 408.5 instead of 406.4 ms).
+// above, the tallest group's runs just before its rows are hashed.  Together
+// against separately, 12 traces of uneven heights in either field at blowup 2 and
+// 4: 2^22 cells 1.5-2.5% faster, 2^24 0.3-1% faster; from 2^25 to 2^29 within 0.6%
+// either way, and 48 BabyBear traces of 2^30.9 cells 0.5% slower.
 constexpr uint64_t kLdeTogetherCells = 1ull << 24;
 
 pico_status enqueue_commit(pico_ctx* ctx, const CommitPlan& plan, cudaStream_t st, cudaStream_t cst,

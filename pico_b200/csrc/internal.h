@@ -59,14 +59,20 @@ cudaError_t upload_p2_constants(int field, const uint32_t ext[8][16], const uint
 // Tests: let the tensor-core form's waits run out (pico_gpu_test_expire_tensor_waits).
 cudaError_t expire_tensor_waits(int64_t tries);
 // Launches of at least this many states use the tensor-core form (p2_tc.cuh).
-// One permutation of n states, one thread per state against the tensor cores
-// (KoalaBear, host call included): 2^15 23.8 / 29.1 us, 2^16 31.2 / 29.3,
-// 2^17 46.2 / 39.1, 2^20 226 / 160.  Below, the latency of one permutation
-// sets the time, and the table load and product stages make it longer.
+// One permutation of n states, one thread per state against the tensor cores,
+// host call included: KoalaBear 2^15 24.8 / 27.5 us, 2^16 32.2 / 31.8, 3 x 2^15
+// 38.5 / 35.7, 2^20 226 / 158; BabyBear 2^15 27.2 / 29.0, 2^16 37.0 / 35.7, 3 x
+// 2^15 45.8 / 41.7.  The lines cross between 2^15 and 2^16 (3 x 2^14 states: 31.1
+// / 29.4, 35.6 / 32.4); trees have powers of two only.  Below, the latency of one
+// permutation sets the time, and the table load and product stages make it longer.
 constexpr uint64_t kTcMinStates = 1u << 16;
-// Rows of several permutations each: from here on.  16 requests of ~20 small
-// traces took 4.78 ms with 2^16, 4.94 with 2^15, 4.49 with 2^14 and 4.39 with
-// 2^13 (runs of one build differ by 0.15 ms, so the last two are equal).
+// Rows of several permutations each: from here on (below it the 16-lane form,
+// up to 2^16 one thread per row, is the other side).  Tree over rows of 100 / 400
+// columns, other form -> tensor cores: KoalaBear 2^13 rows 273 / 588 -> 254 / 529
+// us, 2^14 285 / 617 -> 263 / 537; BabyBear 2^13 266 / 572 -> 276 / 608, 2^14 322 /
+// 764 -> 287 / 620.  So BabyBear's own line is 2^14; one line for both costs its
+// 2^13-row trees 4-6%.  16 KoalaBear requests of ~20 small traces: 4.39 ms with
+// 2^13, 4.49 with 2^14, 4.94 with 2^15, 4.78 with 2^16 (runs differ by 0.15 ms).
 constexpr uint64_t kTcMinRows = 1u << 13;
 // four_lanes: four threads per state (the latency form).  *expired (pinned host
 // memory) changes if a wait of the tensor-core form ran out: states are void.

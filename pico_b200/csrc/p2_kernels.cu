@@ -484,8 +484,9 @@ __global__ void k_challenger_observe(DevChallenger* ch, const uint32_t* vals, ui
 }
 
 // ---------------------------------------------------------------------------
-// Tensor-core forms (p2_tc.cuh): 128 states per CTA of 128 threads, four CTAs
-// per SM (their 4 x 128 TMEM columns).
+// Tensor-core forms (p2_tc.cuh): groups of 128 threads own 128 states each; a
+// CTA of 512 threads holds four groups, which share the tables, and an SM two
+// CTAs (eight groups of 64 TMEM columns).
 
 __host__ __device__ static inline uint64_t tc_tiles(uint64_t n) { return (n + kTcThreads - 1) / kTcThreads; }
 #define PICO_TC_OPEN(F)                                  \

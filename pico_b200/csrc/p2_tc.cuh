@@ -24,9 +24,10 @@
 //     multiply-accumulates in registers.
 //
 // Bound: the multiplier pipe (hashing 2^17 rows
-// of 64 columns: fmaheavy 57% busy, issue 47%) and the latency of
-// the 24 product stages of a permutation (~280 cycles each alone: barrier,
-// products, commit, read-back), which the eight groups of an SM overlap.
+// of 64 columns: fmaheavy 57% busy, issue 47%) and the latency of the 19
+// (KoalaBear) or 18 (BabyBear) product stages of a permutation, plus one or two
+// for its output (~280 cycles each alone: barrier, products, commit, read-back),
+// which the eight groups of an SM overlap.
 // Layout: the accumulators hold half a layer (32 columns), so that z (32
 // columns) and they are 64 columns, eight groups fill the 512 of an SM, and
 // the second half's products run under the first half's S-boxes; the 32-bit

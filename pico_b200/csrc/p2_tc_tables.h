@@ -8,7 +8,7 @@ namespace pico {
 constexpr uint32_t kTcThreads = 128;  // states per group: M of the MMA, one TMEM lane each
 constexpr uint32_t kTcGroups = 4;      // groups per CTA, sharing the tables
 constexpr uint32_t kTcCtas = 2;        // CTAs per SM
-constexpr uint32_t kTcResident = kTcCtas * 148;  // CTAs of a full wave
+constexpr uint32_t kTcResident = kTcCtas * 148;  // CTAs of a full wave (a B200's 148 SMs; fewer only share unevenly)
 constexpr int kTcBlock = 7;           // partial rounds per block: 7 y words and the constant word fill a 32-byte K step
 constexpr uint32_t kTcCols = 64;      // TMEM columns per group (eight groups fill an SM's 512)
 // TMEM columns of a group: the S-box outputs z of a full round (16 x 64

@@ -228,9 +228,9 @@ __global__ void __launch_bounds__(kQThreads) k_quotient(const __grid_constant__ 
 // as byte offsets.
 //
 // Bound: instruction issue (55% of cycles, 2^21 points x 32 columns) and the
-// latency of the interpreter's dependent steps at 28 warps per SM.  The general form reads a column from 32 lines per warp and
-// instruction, for which the L1 is busy 83% of the time, and dispatches 215
-// instructions where 90 are left here.  KoalaBear, host call included:
+// latency of the interpreter's dependent steps at 28 warps per SM.  The general
+// form reads a column from 32 lines per warp and instruction, for which the L1
+// is busy 83% of the time, and dispatches 215 instructions where 90 are left here.  KoalaBear, host call included:
 // 2^20 points x 33 columns 591 -> 345 us, 2^19 x 100 354 -> 290, 2^11 x 8 132 -> 106.
 template <class F>
 __global__ void __launch_bounds__(kQThreads) k_quotient_staged(const __grid_constant__ QuotientArgs A,
