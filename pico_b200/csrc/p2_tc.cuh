@@ -397,7 +397,6 @@ struct P2Tc {
   // Set-up and tear-down, by the whole CTA: tables into shared memory, TMEM
   // columns, a barrier per group, the constant word.
   __device__ __forceinline__ void open(uint8_t* tables, uint64_t* mbar, uint32_t* tmem_slot) {
-    grid_release();
     const uint4* src = g_p2_tc[F::ID];
     for (uint32_t i = threadIdx.x; i < kTcTableBytes / 16; i += kTcThreads * kTcGroups)
       reinterpret_cast<uint4*>(tables)[i] = __ldg(src + i);
@@ -426,6 +425,9 @@ struct P2Tc {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    // Only now: a successor's CTAs hold TMEM while they wait for this kernel, so
+    // every CTA of it has its own first.
+    grid_release();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     tmem = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(tmem_slot), 0) + kTcCols * group;
     lane = tmem + ((warp % 4) << 21);

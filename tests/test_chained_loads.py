@@ -86,3 +86,11 @@ def test_chained_kernels_wait_for_the_kernel_before_them():
             assert re.search(r"lane_load_tables<F>\(|PICO_TC_OPEN\(", body), name
     for waits in ("lane_load_tables", "open"):
         assert all("grid_wait()" in body for body in functions[waits]), waits
+
+
+def test_tensor_memory_is_taken_before_a_successor_may_start():
+    # a waiting successor holds tensor memory: with its own still to come, a CTA
+    # could wait for columns that are given back only after it has finished
+    body, = _functions(_sources())["open"]
+    taken = body.index("__syncthreads()", body.index("tcgen05.alloc"))
+    assert taken < body.index("grid_release()") < body.index("grid_wait()")
